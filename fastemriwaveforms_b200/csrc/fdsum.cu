@@ -17,7 +17,9 @@
 // device (k_fd_extrema, k_fd_bins); a prefix over their bin counts turns the
 // ragged work into one flat bin index space, which k_fd_sum splits into equal
 // contiguous slices, one per warp (lanes take consecutive bins, so the
-// waveform atomics of a warp hit consecutive addresses).  FP64 throughout.
+// waveform atomics of a warp hit consecutive addresses).  What the bins of a
+// (mode, segment) share is formed once, and a bin's root is found directly
+// wherever the general path must find the same one.  FP64 throughout.
 //
 // Numerics follow the reference operation by operation (Cardano roots with the
 // principal complex branches, the same complex arithmetic, the SPA series) so
@@ -29,6 +31,7 @@
 #include <cmath>
 #include <cstdint>
 
+#include "few_common.cuh"
 #include "few_internal.h"
 
 namespace few {
@@ -181,17 +184,39 @@ struct SpaConsts {
     double sixth_s, sixth_c;  // sincos((1/6) pi)
 };
 
-__device__ __forceinline__ SpaConsts spa_consts() {
-    SpaConsts k;
-    k.e23 = cexp_(cdivr(cscale(mk(0.0, 1.0), -2.0 * kPi), 3.0));
-    k.e13 = cexp_(cdivr(cscale(mk(0.0, 1.0), -kPi), 3.0));
-    k.e34 = cexp_(cscale(cscale(mk(-0.0, -1.0), 0.75), kPi));
-    k.sqrt_half_pi = sqrt(0.5 * kPi);
-    const double pi_arg = atan2(0.0, -1.0);
-    sincos(pi_arg / 2.0, &k.half_s, &k.half_c);
-    sincos(__dmul_rn(1.0 / 3.0, pi_arg), &k.third_s, &k.third_c);
-    sincos(__dmul_rn(1.0 / 6.0, pi_arg), &k.sixth_s, &k.sixth_c);
-    return k;
+// Fills the constants and Cardano's xi = (-1 + sqrt(-3)) / 2, one sine and
+// cosine per lane of a CTA's first warp (one after the other on one thread they
+// took most of a short sum: 0.17 ms for 1.2 million bins).  The exponentials are
+// of purely imaginary arguments (exp(+-0) = 1) and the angle of -3 + 0i is pi.
+__device__ __forceinline__ void spa_consts(SpaConsts &k, cx &xi) {
+    const int lane = threadIdx.x;
+    if (lane >= 6) return;
+    const double angle = lane == 0   ? -2.0 * kPi / 3.0
+                         : lane == 1 ? -kPi / 3.0
+                         : lane == 2 ? __dmul_rn(-0.75, kPi)
+                         : lane == 3 ? kPi / 2.0
+                         : lane == 4 ? __dmul_rn(1.0 / 3.0, kPi)
+                                     : __dmul_rn(1.0 / 6.0, kPi);
+    double s, c;
+    sincos(angle, &s, &c);
+    if (lane == 0) k.e23 = mk(c, s);
+    if (lane == 1) k.e13 = mk(c, s);
+    if (lane == 2) k.e34 = mk(c, s);
+    if (lane == 3) {
+        k.half_s = s;
+        k.half_c = c;
+        const double rho = sqrt(3.0);
+        xi = mk((-1.0 + __dmul_rn(rho, c)) / 2.0, __dmul_rn(rho, s) / 2.0);
+    }
+    if (lane == 4) {
+        k.third_s = s;
+        k.third_c = c;
+        k.sqrt_half_pi = sqrt(0.5 * kPi);
+    }
+    if (lane == 5) {
+        k.sixth_s = s;
+        k.sixth_c = c;
+    }
 }
 
 // csqrt_(r + 0i): the same bits without atan2 and sincos.
@@ -512,92 +537,448 @@ __device__ __forceinline__ void red_add(double2 *p, cx v) {
     atomicAdd(&p->y, v.im);
 }
 
+// One (mode, segment, bin) evaluation in the reference's operations: Cardano's
+// roots and the stationary-phase term of each root inside the segment.
+__device__ __forceinline__ void fd_bin(const SumArgs &A, const SpaConsts &SK, const cx &xi, int mode, int seg,
+                                       int i) {
+    const int m = A.m[mode], k = A.k[mode], n = A.n[mode];
+    const double f = A.freq[i];
+    // mode-frequency cubic on this segment
+    const double *fy = A.fco + (long long)seg * A.fj;
+    double fyv = m * fy[0] + k * fy[A.fp] + n * fy[2 * A.fp];
+    double fc1 = m * fy[A.fq] + k * fy[A.fq + A.fp] + n * fy[A.fq + 2 * A.fp];
+    double fc2 = m * fy[2 * A.fq] + k * fy[2 * A.fq + A.fp] + n * fy[2 * A.fq + 2 * A.fp];
+    double fc3 = m * fy[3 * A.fq] + k * fy[3 * A.fq + A.fp] + n * fy[3 * A.fq + 2 * A.fp];
+    double roots[3];
+    cube_roots(fc3, fc2, fc1, fyv - f, xi, roots, SK);
+    const double ts = A.t[seg], te = A.t[seg + 1];
+    for (int r = 0; r < 3; ++r) {
+        double x = roots[r];
+        double tt = ts + x;
+        if (!(tt < te && tt >= ts)) continue;
+        double x2 = x * x, x3 = x * x2;
+        const double *ar = A.amp + (long long)mode * A.ap + (long long)seg * A.aj;
+        const double *ai = ar + (long long)A.K * A.ap;
+        double Rre = ar[0] + ar[A.aq] * x + ar[2 * A.aq] * x2 + ar[3 * A.aq] * x3;
+        double Rim = ai[0] + ai[A.aq] * x + ai[2 * A.aq] * x2 + ai[3 * A.aq] * x3;
+        double h = A.phase_t[seg + 1] - A.phase_t[seg];
+        double s = (tt - A.phase_t[seg]) / h;
+        double s1 = 1.0 - s, s2 = s * s, s3 = s * s2, s4 = s * s3, s5 = s * s4;
+        double h2 = h * h, h3 = h * h2;
+        double phase = 0.0, fdot = 0.0, fddot = 0.0;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const int mult = q == 0 ? m : (q == 1 ? k : n);
+            const double *c = A.pc + (long long)q * A.pcf + (long long)seg * A.pcs;
+            double c0 = c[0], c1 = c[A.pcc], c2 = c[2 * A.pcc], c3 = c[3 * A.pcc];
+            double c4 = c[4 * A.pcc], c5 = c[5 * A.pcc], c6 = c[6 * A.pcc], c7 = c[7 * A.pcc];
+            double P = c0 + s * (c1 + s1 * (c2 + s * (c3 + s1 * (c4 + s * (c5 + s1 * (c6 + s * c7))))));
+            double d2 = (-2. * c2 + c3 * (2. - 6. * s) + c4 * (2. - 12. * s + 12. * s2) +
+                         c5 * (6. * s - 24. * s2 + 20. * s3) + c6 * (6. * s - 36. * s2 + 60. * s3 - 30. * s4) +
+                         c7 * (12. * s2 - 60. * s3 + 90. * s4 - 42. * s5)) /
+                        (2. * kPi * h2);
+            double d3 = (-6. * c3 + c4 * (-12. + 24. * s) + c5 * (6. - 48. * s + 60. * s2) +
+                         c6 * (6. - 72. * s + 180. * s2 - 120. * s3) +
+                         c7 * (24. * s - 180. * s2 + 360. * s3 - 210. * s4)) /
+                        (2. * kPi * h3);
+            if (q == 0) { phase = mult * P; fdot = mult * d2; fddot = mult * d3; }
+            else { phase += mult * P; fdot += mult * d2; fddot += mult * d3; }
+        }
+        double arg = 2. * kPi * fdot * fdot * fdot / (3. * fddot * fddot);
+        double pre = -1.0 * fdot / fabs(fddot) * 2. / sqrt(3.);
+        cx amp2 = cdiv(cscale(spa(arg, SK), pre), csqrt_real(arg, SK));
+        double ph = 2. * kPi * f * tt - phase;
+        cx te_ = cmul(cmul(mk(Rre, Rim), amp2), cexp_i(ph));
+        double2 yp = A.ylms[mode];
+        red_add(A.wf + i, cmul(mk(yp.x, yp.y), te_));
+        if (m != 0 && A.include_minus_m) {
+            int im = 2 * A.zero_index - i;
+            if (im >= 0 && im < A.L) {
+                double2 ym = A.ylms[A.K + mode];
+                red_add(A.wf + im, cmul(mk(ym.x, ym.y), cconj(te_)));
+            }
+        }
+    }
+}
+
+__device__ __noinline__ void fd_bin_general(const SumArgs &A, const SpaConsts &SK, const cx &xi, int mode, int seg,
+                                            int i) {
+    fd_bin(A, SK, xi, mode, seg, i);
+}
+
+// (mode, segment) of entry e = mode * nseg + seg.
+__device__ __forceinline__ void mode_seg(const SumArgs &A, long long e, int &mode, int &seg) {
+    const unsigned nseg = A.N - 1;
+    if (A.E <= 0xffffffffLL) {  // a 64-bit division costs about 100 instructions
+        const unsigned q = (unsigned)e / nseg;
+        mode = (int)q;
+        seg = (int)((unsigned)e - q * nseg);
+    } else {
+        mode = (int)(e / nseg);
+        seg = (int)(e % nseg);
+    }
+}
+
+// What the bins of one (mode, segment) entry share, formed once per entry.
+struct Entry {
+    double c0, c1, c2, c3;        // mode-frequency cubic in x = t - t_seg
+    double tc2, tc3;              // 2 c2, 3 c3
+    double ic1, g2, g3;           // first guess of the root: w (1 + w (g2 + w g3)), w = (f - c0) / c1
+    double lo, hi;                // the direct root is taken when lo <= x <= hi (none when lo > hi)
+    double bc;                    // c2 / c3
+    double pair_lo, pair_hi;      // and bc + x lies outside [pair_lo, pair_hi]
+    double ts, pt, h, ih;         // segment start, phase knot, phase step and its reciprocal
+    double pphi[8], pr[8];        // Phi_phi, Phi_r in the 8-term basis
+    double d2[6];                 // fdot = sum_j d2[j] s^j (all fields, over 2 pi h^2)
+    double a[8];                  // amplitude cubic, real then imaginary part
+    double m, k, n;
+    double ypx, ypy, ymx, ymy;    // Y+, Y- (Y- unused when minus = 0)
+    int off;                      // bin index of the batch's flat bin b is b + off
+    int mode, seg;
+    int minus;
+};
+constexpr int kBatch = 16;  // entries a warp holds at a time
+constexpr int kSumThreads = 128;
+// Fewer bins per entry than this on average and forming the entries costs more
+// than it saves (general path for every bin against entries: 0.88 and 1.13 ms at
+// 3.6, 0.33 and 0.40 ms at 6.5, 1.80 and 1.36 ms at 10.1 bins per entry).
+constexpr long long kMinBins = 10;
+constexpr long long kMinSlice = 64;  // bins a warp takes at least (its CTA's constants and entries serve them)
+
+// Bound on the error of Cardano's root as the general path computes it, as a
+// share of the segment's length.  alpha, beta: the cubic and quadratic terms
+// over the linear one at the segment's far end, d0 = beta^2 - 3 alpha (signed).
+// Terms: the sum b + C + D0/C (beta/alpha); the angle of C when S << D1
+// (beta^3/alpha^2); C itself when beta^2 << alpha (alpha^-1/2); and z = S + D1
+// when D0^3 << D1^2.  The factor takes in the rounding of exp(log(z)/3) at
+// |log z| ~ 150; over 24 million sampled roots the error reached 0.75 of it.
+// Single precision: the bound's own size matters to a few per cent, and what
+// under- or overflows gives infinity or NaN, which no test below accepts.
+__device__ __forceinline__ float cardano_error(float alpha, float beta, float d0) {
+    const float dm = 2.0f * beta * beta * beta + 9.0f * alpha * beta + 40.0f * alpha * alpha;
+    const float ba = __fdividef(beta, alpha), ad0 = fabsf(d0);
+    const float z = fmaxf(__fdividef(dm * dm, ad0 * ad0 * ad0), 4.0f);
+    return 1.1e-14f * (1.0f + ba + ba * ba * beta + rsqrtf(alpha) + __fdividef(exp2f(__log2f(dm) * (1.0f / 3.0f)), alpha) * z);
+}
+
+// 1/a to 20 bits (the hardware's approximation).
+__device__ __forceinline__ double rcp_approx(double a) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(a));
+    return r;
+}
+
+__device__ __forceinline__ void fill_entry(const SumArgs &A, long long e, long long base, Entry &E) {
+    int mode, seg;
+    mode_seg(A, e, mode, seg);
+    const int m = A.m[mode], k = A.k[mode], n = A.n[mode];
+    const double *fy = A.fco + (long long)seg * A.fj;
+    E.c0 = m * fy[0] + k * fy[A.fp] + n * fy[2 * A.fp];
+    E.c1 = m * fy[A.fq] + k * fy[A.fq + A.fp] + n * fy[A.fq + 2 * A.fp];
+    E.c2 = m * fy[2 * A.fq] + k * fy[2 * A.fq + A.fp] + n * fy[2 * A.fq + 2 * A.fp];
+    E.c3 = m * fy[3 * A.fq] + k * fy[3 * A.fq + A.fp] + n * fy[3 * A.fq + 2 * A.fp];
+    E.tc2 = 2.0 * E.c2;
+    E.tc3 = 3.0 * E.c3;
+    E.ts = A.t[seg];
+    const double H = A.t[seg + 1] - E.ts;
+    const double rc1 = rcp_approx(E.c1);
+    E.ic1 = fma(fma(-E.c1, rc1, 1.0), rc1, rc1);
+    E.g2 = -E.c2 * E.ic1;
+    E.g3 = 2.0 * E.g2 * E.g2 - E.c3 * E.ic1;
+    E.bc = E.c2 * rcp_approx(E.c3);
+    E.pair_lo = -2.2 * H;
+    E.pair_hi = 0.2 * H;
+    // The cubic is monotonic on [-H, 2H] when its slope varies by less than
+    // c1 there, so a root in the segment is the only real one near it; the
+    // other two then have real parts -(c2/c3 + x)/2.
+    const double ic1 = fabs(E.ic1);
+    const float alpha = (float)(fabs(E.c3) * H * H * ic1), beta = (float)(fabs(E.c2) * H * ic1);
+    const float d0 = beta * beta - ((E.c3 > 0.0) == (E.c1 > 0.0) ? 3.0f : -3.0f) * alpha;
+    const float err = cardano_error(alpha, beta, d0);
+    const bool direct = 4.0f * beta + 12.0f * alpha < 1.0f && err < 1e-6f;
+    const double margin = 8.0 * err * H + 1e-15 * (fabs(E.ts) + H);  // the second term: the rounding of t_seg + x
+    E.lo = direct ? margin : 1.0;
+    E.hi = direct ? H - margin : -1.0;
+    E.pt = A.phase_t[seg];
+    E.h = A.phase_t[seg + 1] - E.pt;
+    E.ih = 1.0 / E.h;
+    double c[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const double mult = q == 0 ? m : (q == 1 ? k : n);
+        const double *pc = A.pc + (long long)q * A.pcf + (long long)seg * A.pcs;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const double v = pc[j * A.pcc];
+            if (q == 0) E.pphi[j] = v;
+            if (q == 2) E.pr[j] = v;
+            c[j] = fma(mult, v, c[j]);
+        }
+    }
+    // second derivative of the 8-term basis, by powers of s
+    const double w = E.ih * E.ih / (2. * kPi);
+    E.d2[0] = w * (-2. * c[2] + 2. * c[3] + 2. * c[4]);
+    E.d2[1] = w * (-6. * c[3] - 12. * c[4] + 6. * c[5] + 6. * c[6]);
+    E.d2[2] = w * (12. * c[4] - 24. * c[5] - 36. * c[6] + 12. * c[7]);
+    E.d2[3] = w * (20. * c[5] + 60. * c[6] - 60. * c[7]);
+    E.d2[4] = w * (-30. * c[6] + 90. * c[7]);
+    E.d2[5] = w * (-42. * c[7]);
+    const double *ar = A.amp + (long long)mode * A.ap + (long long)seg * A.aj;
+    const double *ai = ar + (long long)A.K * A.ap;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        E.a[q] = ar[q * A.aq];
+        E.a[4 + q] = ai[q * A.aq];
+    }
+    E.m = m;
+    E.k = k;
+    E.n = n;
+    const double2 yp = A.ylms[mode], ym = A.ylms[A.K + mode];
+    E.ypx = yp.x;
+    E.ypy = yp.y;
+    E.ymx = ym.x;
+    E.ymy = ym.y;
+    E.minus = m != 0 && A.include_minus_m;
+    E.mode = mode;
+    E.seg = seg;
+    E.off = (int)(A.lo[e] + (base - A.prefix[e]));
+}
+
+// 1/sqrt(a) for a normal a: the hardware's approximation (20 bits) and one step
+// of the third-order iteration (error 2^-60 before rounding).
+__device__ __forceinline__ double rsqrt_pos(double a) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+    const double e = fma(-a * y, y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// The general path's values from NB roots x found directly, for |SPA argument|
+// > 7.  With q = fdot / fddot the argument is (2 pi / 3) fdot q^2, and the
+// factor pre / sqrt(argument) collapses to -sign(fdot) sqrt(2 / pi) / sqrt|fdot|
+// (times -i when the argument is negative), so one reciprocal square root
+// serves the amplitude and the asymptotic series' 1/argument.  The phase keeps
+// the general path's operations, since its rounding (at ~1e7 rad) shows in the
+// result.  ok is cleared where the argument is not large.
+template <int NB>
+__device__ __forceinline__ void fd_terms_direct(const SumArgs &A, const Entry &E, const double (&f)[NB],
+                                                const double (&x)[NB], bool (&ok)[NB], cx (&term)[NB]) {
+    double s[NB], s1[NB], tt[NB], phase[NB], P[NB];
+    cx amp[NB];
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        tt[q] = E.ts + x[q];
+        const double u = tt[q] - E.pt;
+        const double v = u * E.ih;
+        s[q] = fma(fma(-v, E.h, u), E.ih, v);  // u / h rounded
+        s1[q] = 1.0 - s[q];
+    }
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        double fdot = E.d2[5], fdd = E.d2[5];
+#pragma unroll
+        for (int j = 4; j >= 1; --j) {
+            fdot = fma(fdot, s[q], E.d2[j]);
+            fdd = fma(fdd, s[q], fdot);
+        }
+        fdot = fma(fdot, s[q], E.d2[0]);
+        fdd *= E.ih;
+        const double rs = rsqrt_pos(fabs(fdot)), ri = rs * rs;  // |fdot|^{-1/2}, 1/|fdot|
+        const double g = fdd * ri;
+        double y = 1.5 / kPi * (g * g) * ri;  // 1 / |argument|
+        ok[q] = ok[q] && y < 1.0 / 7.0 && fdd != 0.0 && rs < 1e300;
+        const bool neg = fdot < 0.0;
+        if (neg) y = -y;
+        const double y2 = y * y;
+        const double sim =
+            fma(fma(fma(fma(c_spa.ai[8], y2, c_spa.ai[6]), y2, c_spa.ai[4]), y2, c_spa.ai[2]), y2, c_spa.ai[0]);
+        const double sre = y * fma(fma(fma(c_spa.ar[7], y2, c_spa.ar[5]), y2, c_spa.ar[3]), y2, c_spa.ar[1]);
+        // e^{-3 pi i/4} sqrt(pi/2) (sre + i sim) x (-sign sqrt(2/pi)) = +-sqrt(1/2) (1 + i)(sre + i sim)
+        const double kHalfSqrt = 0.70710678118654752440;
+        const double w = (neg ? -kHalfSqrt : kHalfSqrt) * rs;
+        const double qre = w * (sre - sim), qim = w * (sre + sim);
+        const cx amp2 = neg ? mk(qim, -qre) : mk(qre, qim);
+        const double Rre = fma(fma(fma(E.a[3], x[q], E.a[2]), x[q], E.a[1]), x[q], E.a[0]);
+        const double Rim = fma(fma(fma(E.a[7], x[q], E.a[6]), x[q], E.a[5]), x[q], E.a[4]);
+        amp[q] = cmul(mk(Rre, Rim), amp2);
+    }
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        P[q] = E.pphi[7];
+#pragma unroll
+        for (int j = 6; j >= 0; --j) P[q] = fma((j & 1) ? s1[q] : s[q], P[q], E.pphi[j]);
+        phase[q] = E.m * P[q];
+    }
+    if (E.k != 0.0) {
+        const double *t = A.pc + A.pcf + (long long)E.seg * A.pcs;
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+            P[q] = t[7 * A.pcc];
+#pragma unroll
+            for (int j = 6; j >= 0; --j) P[q] = fma((j & 1) ? s1[q] : s[q], P[q], t[j * A.pcc]);
+            phase[q] = fma(E.k, P[q], phase[q]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        P[q] = E.pr[7];
+#pragma unroll
+        for (int j = 6; j >= 0; --j) P[q] = fma((j & 1) ? s1[q] : s[q], P[q], E.pr[j]);
+        phase[q] = fma(E.n, P[q], phase[q]);
+        const double ph = fma(2. * kPi * f[q], tt[q], -phase[q]);
+        ok[q] = ok[q] && fabs(ph) < kPhaseMax;
+        double sn, cs;
+        sincos_phase_core(ph, &sn, &cs);
+        term[q] = cmul(amp[q], mk(cs, sn));
+    }
+}
+
+// NB bins of one entry on each lane: i the bin indices, live the lanes' bins
+// that exist.
+template <int NB>
+__device__ __forceinline__ void fd_bins(const SumArgs &A, const Entry &E, const int (&i)[NB], const double (&f)[NB],
+                                        const bool (&live)[NB], const SpaConsts &SK, const cx &xi) {
+    double x[NB], d[NB];
+    bool direct[NB];
+    const double tol = 1e-9 * E.hi;
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        d[q] = E.c0 - f[q];
+        const double g = -d[q] * E.ic1;
+        x[q] = g * fma(g, fma(g, E.g3, E.g2), 1.0);
+        direct[q] = E.lo <= E.hi && x[q] > -0.5 * E.hi && x[q] < 1.5 * E.hi;
+    }
+    for (int it = 0; it < 6; ++it) {
+        bool more = false;
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+            const double p = fma(fma(fma(E.c3, x[q], E.c2), x[q], E.c1), x[q], d[q]);
+            const double dp = fma(fma(E.tc3, x[q], E.tc2), x[q], E.c1);
+            const double dx = p * rcp_approx(dp);
+            x[q] -= dx;
+            const bool far = direct[q] && !(fabs(dx) <= tol);
+            more = more || far;
+            if (it == 5 && far) direct[q] = false;
+        }
+        if (!__any_sync(0xffffffffu, more)) break;
+    }
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        const double pr = E.bc + x[q];
+        direct[q] = direct[q] && x[q] >= E.lo && x[q] <= E.hi && (pr < E.pair_lo || pr > E.pair_hi);
+    }
+    cx term[NB];
+    fd_terms_direct(A, E, f, x, direct, term);
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        if (live[q] && direct[q]) {
+            red_add(A.wf + i[q], cmul(mk(E.ypx, E.ypy), term[q]));
+            const int im = 2 * A.zero_index - i[q];
+            if (E.minus && im >= 0 && im < A.L) red_add(A.wf + im, cmul(mk(E.ymx, E.ymy), cconj(term[q])));
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < NB; ++q)
+        if (live[q] && !direct[q]) fd_bin_general(A, SK, xi, E.mode, E.seg, i[q]);
+}
+
+// The flat bins are cut into equal contiguous slices, one per warp; a warp
+// takes the entries of its slice kBatch at a time, forms what their bins share
+// (lane = entry) into shared memory, and then evaluates the bins (lane =
+// consecutive bin; two bins 32 apart on a lane while every lane's two belong to
+// one entry, which halves the shared-memory reads).  A bin's root comes from
+// Newton's iteration when the entry's cubic is monotonic around the segment and
+// the root lies inside it by more than Cardano's rounding error could move it,
+// so that the general path would find the same single root there; every other
+// bin (the segment's ends, turnovers, small SPA arguments: 0.4 to 8 % of them)
+// takes the general path.
+// Bound by the FP64 pipe's latency and the shared-memory reads together (FP64
+// pipe 48 % busy, issue slots 59 % at 16 warps per SM).  One year, 3843 modes,
+// 889 million (mode, bin) evaluations: 15.0 ms; 65.7 ms with every bin on the
+// general path (1390 instructions a bin against about 320), 17.2 ms with one bin
+// a lane, 26.1 ms at 8 warps per SM.
 template <int MINB>
-__global__ void __launch_bounds__(256, MINB) k_fd_sum(SumArgs A) {
+__global__ void __launch_bounds__(kSumThreads, MINB) k_fd_sum(const __grid_constant__ SumArgs A) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     const long long B = A.prefix[A.E];
-    const long long W = (long long)gridDim.x * (blockDim.x >> 5);
+    const bool sparse = B < kMinBins * A.E;
+    long long W = (long long)gridDim.x * (blockDim.x >> 5);
+    if (W > B / kMinSlice + 1) W = B / kMinSlice + 1;
     const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
-    const long long b0 = B * w / W, b1 = B * (w + 1) / W;
+    const long long b0 = w < W ? B * w / W : B, b1 = w < W ? B * (w + 1) / W : B;
     // run-time constants of the SPA function and of Cardano's formula, once per
     // CTA in shared memory (they would hold 18 registers for the whole kernel)
     __shared__ SpaConsts s_sk;
     __shared__ cx s_xi;
-    if (threadIdx.x == 0) {
-        s_sk = spa_consts();
-        s_xi = cdivr(cadd(mk(-1.0, 0.0), csqrt_(mk(-3.0, 0.0))), 2.0);
-    }
+    if ((long long)blockIdx.x * (blockDim.x >> 5) >= W) return;
+    spa_consts(s_sk, s_xi);
     __syncthreads();
     if (b0 >= b1) return;
-    const SpaConsts &SK = s_sk;
-    const cx &xi = s_xi;
-    const int nseg = A.N - 1;
-    long long e = find_entry(A.prefix, 0, A.E - 1, b0 + lane < b1 ? b0 + lane : b1 - 1);
-    for (long long base = b0; base < b1; base += 32) {
-        long long b = base + lane;
-        if (b >= b1) break;
-        e = advance_entry(A.prefix, A.E, e, b);
-        int i = A.lo[e] + (int)(b - A.prefix[e]);
-        int mode = (int)(e / nseg), seg = (int)(e % nseg);
-        int m = A.m[mode], k = A.k[mode], n = A.n[mode];
-        double f = A.freq[i];
-        // mode-frequency cubic on this segment
-        const double *fy = A.fco + (long long)seg * A.fj;
-        double fyv = m * fy[0] + k * fy[A.fp] + n * fy[2 * A.fp];
-        double fc1 = m * fy[A.fq] + k * fy[A.fq + A.fp] + n * fy[A.fq + 2 * A.fp];
-        double fc2 = m * fy[2 * A.fq] + k * fy[2 * A.fq + A.fp] + n * fy[2 * A.fq + 2 * A.fp];
-        double fc3 = m * fy[3 * A.fq] + k * fy[3 * A.fq + A.fp] + n * fy[3 * A.fq + 2 * A.fp];
-        double roots[3];
-        cube_roots(fc3, fc2, fc1, fyv - f, xi, roots, SK);
-        const double ts = A.t[seg], te = A.t[seg + 1];
-        for (int r = 0; r < 3; ++r) {
-            double x = roots[r];
-            double tt = ts + x;
-            if (!(tt < te && tt >= ts)) continue;
-            double x2 = x * x, x3 = x * x2;
-            const double *ar = A.amp + (long long)mode * A.ap + (long long)seg * A.aj;
-            const double *ai = ar + (long long)A.K * A.ap;
-            double Rre = ar[0] + ar[A.aq] * x + ar[2 * A.aq] * x2 + ar[3 * A.aq] * x3;
-            double Rim = ai[0] + ai[A.aq] * x + ai[2 * A.aq] * x2 + ai[3 * A.aq] * x3;
-            double h = A.phase_t[seg + 1] - A.phase_t[seg];
-            double s = (tt - A.phase_t[seg]) / h;
-            double s1 = 1.0 - s, s2 = s * s, s3 = s * s2, s4 = s * s3, s5 = s * s4;
-            double h2 = h * h, h3 = h * h2;
-            double phase = 0.0, fdot = 0.0, fddot = 0.0;
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                const int mult = q == 0 ? m : (q == 1 ? k : n);
-                const double *c = A.pc + (long long)q * A.pcf + (long long)seg * A.pcs;
-                double c0 = c[0], c1 = c[A.pcc], c2 = c[2 * A.pcc], c3 = c[3 * A.pcc];
-                double c4 = c[4 * A.pcc], c5 = c[5 * A.pcc], c6 = c[6 * A.pcc], c7 = c[7 * A.pcc];
-                double P = c0 + s * (c1 + s1 * (c2 + s * (c3 + s1 * (c4 + s * (c5 + s1 * (c6 + s * c7))))));
-                double d2 = (-2. * c2 + c3 * (2. - 6. * s) + c4 * (2. - 12. * s + 12. * s2) +
-                             c5 * (6. * s - 24. * s2 + 20. * s3) + c6 * (6. * s - 36. * s2 + 60. * s3 - 30. * s4) +
-                             c7 * (12. * s2 - 60. * s3 + 90. * s4 - 42. * s5)) /
-                            (2. * kPi * h2);
-                double d3 = (-6. * c3 + c4 * (-12. + 24. * s) + c5 * (6. - 48. * s + 60. * s2) +
-                             c6 * (6. - 72. * s + 180. * s2 - 120. * s3) +
-                             c7 * (24. * s - 180. * s2 + 360. * s3 - 210. * s4)) /
-                            (2. * kPi * h3);
-                if (q == 0) { phase = mult * P; fdot = mult * d2; fddot = mult * d3; }
-                else { phase += mult * P; fdot += mult * d2; fddot += mult * d3; }
-            }
-            double arg = 2. * kPi * fdot * fdot * fdot / (3. * fddot * fddot);
-            double pre = -1.0 * fdot / fabs(fddot) * 2. / sqrt(3.);
-            cx amp2 = cdiv(cscale(spa(arg, SK), pre), csqrt_real(arg, SK));
-            double ph = 2. * kPi * f * tt - phase;
-            cx te_ = cmul(cmul(mk(Rre, Rim), amp2), cexp_i(ph));
-            double2 yp = A.ylms[mode];
-            red_add(A.wf + i, cmul(mk(yp.x, yp.y), te_));
-            if (m != 0 && A.include_minus_m) {
-                int im = 2 * A.zero_index - i;
-                if (im >= 0 && im < A.L) {
-                    double2 ym = A.ylms[A.K + mode];
-                    red_add(A.wf + im, cmul(mk(ym.x, ym.y), cconj(te_)));
-                }
-            }
+    if (sparse) {
+        long long e = find_entry(A.prefix, 0, A.E - 1, b0 + lane < b1 ? b0 + lane : b1 - 1);
+        for (long long b = b0 + lane; b < b1; b += 32) {
+            e = advance_entry(A.prefix, A.E, e, b);
+            int mode, seg;
+            mode_seg(A, e, mode, seg);
+            fd_bin(A, s_sk, s_xi, mode, seg, A.lo[e] + (int)(b - A.prefix[e]));
         }
+        return;
     }
+    Entry *ent = reinterpret_cast<Entry *>(smem_raw) + (threadIdx.x >> 5) * kBatch;
+    __shared__ int s_end[kSumThreads / 32][kBatch];
+    int *end = s_end[threadIdx.x >> 5];  // ends of the batch's entries, from its first bin
+    long long e = find_entry(A.prefix, 0, A.E - 1, b0);
+    for (long long base = b0; base < b1;) {
+        __syncwarp();
+        if (lane < kBatch) {
+            const long long q = e + lane;
+            const long long last = A.prefix[q + 1 < A.E ? q + 1 : A.E];
+            end[lane] = (int)((last < b1 ? last : b1) - base);
+            if (q < A.E && last > A.prefix[q]) fill_entry(A, q, base, ent[lane]);
+        }
+        __syncwarp();
+        const int stop = end[kBatch - 1];
+        int slot = 0;
+        for (int at = 0; at < stop;) {
+            int b[2], sl[2], i[2];
+            double f[2];
+            bool live[2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                b[q] = at + 32 * q + lane;
+                live[q] = b[q] < stop;
+                b[q] = live[q] ? b[q] : stop - 1;
+                while (end[slot] <= b[q]) ++slot;
+                sl[q] = slot;
+                i[q] = b[q] + ent[slot].off;
+                f[q] = A.freq[i[q]];
+            }
+            if (__all_sync(0xffffffffu, sl[0] == sl[1])) {
+                fd_bins<2>(A, ent[sl[0]], i, f, live, s_sk, s_xi);
+                at += 64;
+            } else {
+                const int i1[1] = {i[0]};
+                const double f1[1] = {f[0]};
+                const bool live1[1] = {live[0]};
+                fd_bins<1>(A, ent[sl[0]], i1, f1, live1, s_sk, s_xi);
+                slot = sl[0];
+                at += 32;
+            }
+            __syncwarp();
+        }
+        base += stop;
+        if (base < b1) e = advance_entry(A.prefix, A.E, e + kBatch - 1 < A.E ? e + kBatch - 1 : A.E - 1, base);
+    }
+}
+
+template <int MINB>
+int launch_fd_sum(const SumArgs &A, int blocks, cudaStream_t st) {
+    const int smem = kSumThreads / 32 * kBatch * (int)sizeof(Entry);
+    FEW_CUDA_TRY(ensure_smem_attr((const void *)k_fd_sum<MINB>, smem));
+    k_fd_sum<MINB><<<blocks * (256 / kSumThreads), kSumThreads, smem, st>>>(A);
+    FEW_LAUNCH_CHECK("k_fd_sum");
+    return FEW_OK;
 }
 
 // (h+, hx) from the two-sided spectrum (fdinterp.py:518-536):
@@ -782,19 +1163,17 @@ extern "C" FEW_API int few_fd_sum(void *wf, int L, const double *freq, int zero_
     A.lo = lo;
     A.prefix = prefix;
     A.E = (long long)K * (N - 1);
-    // ctas_per_sm selects the register budget of the kernel (1: 255, 2: 128,
-    // 3: 80 registers a thread); blocks is the grid (0: 32 CTAs per SM: the
-    // static slices of the bin space are short enough that the last warps to
-    // finish trail by little; measured 83.9 ms against 85.6 ms at 8 per SM on
-    // the one-year, 3843-mode case).
+    // ctas_per_sm selects the register budget of the kernel (1: 148, 2: 128, 3: 96
+    // registers a thread: 16.3, 15.0 and 15.3 ms on the one-year, 3843-mode case);
+    // blocks is the grid in units of 256 threads (0: 32 per SM: the static slices
+    // of the bin space are short enough that the last warps to finish trail by
+    // little).
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (blocks <= 0) blocks = 148 * 32;
     if (ctas_per_sm <= 0) ctas_per_sm = 2;
-    if (ctas_per_sm == 1) few::fd::k_fd_sum<1><<<blocks, 256, 0, st>>>(A);
-    else if (ctas_per_sm == 3) few::fd::k_fd_sum<3><<<blocks, 256, 0, st>>>(A);
-    else few::fd::k_fd_sum<2><<<blocks, 256, 0, st>>>(A);
-    FEW_LAUNCH_CHECK("k_fd_sum");
-    return FEW_OK;
+    if (ctas_per_sm == 1) return few::fd::launch_fd_sum<2>(A, blocks, st);
+    if (ctas_per_sm == 3) return few::fd::launch_fd_sum<5>(A, blocks, st);
+    return few::fd::launch_fd_sum<4>(A, blocks, st);
 }
 
 extern "C" FEW_API int few_fd_finalize(const void *wf, int L, int first, int count, void *out, void *stream) {

@@ -84,6 +84,57 @@ __device__ __forceinline__ void sincos_reduced(double ph, double *s, double *c)
     sincos(r, s, c);
 }
 
+// sin and cos of an angle of any size met in a phase (|ph| < kPhaseMax), both to
+// about an ulp: the angle is reduced mod pi/2 by Cody & Waite's method (pi/2 in
+// three parts of 32, 32 and 53 bits; with fused multiply-adds the first
+// difference is exact for every such angle, being a multiple of 2^-31 below 1
+// or of ph's own last place), then Taylor's series on |r| <= pi/4, whose first
+// dropped terms (r^19/19!, r^18/18!) are below 1e-19 and 3e-18.  A third fewer
+// FP64 operations than a reduction mod 2 pi followed by sincos, which reduces
+// again.
+constexpr double kPhaseMax = 1073741824.0;  // 2^30
+
+__device__ __forceinline__ void sincos_phase_core(double ph, double *s, double *c)
+{
+    const double kMagic = 6755399441055744.0;  // 1.5 * 2^52: the sum's low word is the rounded integer
+    const double kC1 = 0x1.921fb54400000p+0, kC2 = 0x1.0b4611a600000p-34, kC3 = 0x1.3198a2e037073p-69;
+    const double km = __fma_rn(ph, 0.63661977236758134, kMagic);
+    const int q = __double2loint(km);
+    const double k = __dsub_rn(km, kMagic);
+    double r = __fma_rn(-k, kC1, ph);
+    r = __fma_rn(-k, kC2, r);
+    r = __fma_rn(-k, kC3, r);
+    const double z = r * r;
+    double p = 1.0 / 355687428096000.0;
+    p = __fma_rn(p, z, -1.0 / 1307674368000.0);
+    p = __fma_rn(p, z, 1.0 / 6227020800.0);
+    p = __fma_rn(p, z, -1.0 / 39916800.0);
+    p = __fma_rn(p, z, 1.0 / 362880.0);
+    p = __fma_rn(p, z, -1.0 / 5040.0);
+    p = __fma_rn(p, z, 1.0 / 120.0);
+    p = __fma_rn(p, z, -1.0 / 6.0);
+    const double sn = __fma_rn(r * z, p, r);
+    double u = 1.0 / 20922789888000.0;
+    u = __fma_rn(u, z, -1.0 / 87178291200.0);
+    u = __fma_rn(u, z, 1.0 / 479001600.0);
+    u = __fma_rn(u, z, -1.0 / 3628800.0);
+    u = __fma_rn(u, z, 1.0 / 40320.0);
+    u = __fma_rn(u, z, -1.0 / 720.0);
+    u = __fma_rn(u, z, 1.0 / 24.0);
+    const double hz = 0.5 * z, w = 1.0 - hz;
+    const double cn = w + __fma_rn(z * z, u, (1.0 - w) - hz);
+    const double a = (q & 1) ? cn : sn, b = (q & 1) ? sn : cn;
+    *s = (q & 2) ? -a : a;
+    *c = ((q + 1) & 2) ? -b : b;
+}
+
+// The same for any angle: larger and non-finite ones go to sincos.
+__device__ __forceinline__ void sincos_phase(double ph, double *s, double *c)
+{
+    if (fabs(ph) < kPhaseMax) sincos_phase_core(ph, s, c);
+    else sincos(ph, s, c);
+}
+
 // The 8-term dense-output phase polynomial in s, s1 = 1 - s, in the
 // operation order of src/few/cutils/interpolate.cu:642-644, every product and
 // sum rounded separately.
