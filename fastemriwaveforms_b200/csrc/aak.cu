@@ -13,17 +13,28 @@
 // sample is (hI, -hII).
 //
 // B200 layout: one launch over all samples (the reference launches one kernel
-// per trajectory segment); a thread finds its segment by bisection over the
-// segments' first samples.  The five Bessel values of a harmonic come from
-// one backward (Miller) recurrence normalised by J_0 + 2 sum J_2k = 1, instead
-// of five separate evaluations; the harmonic phase n Phi (+ Doppler) is formed
-// as the reference forms it (its rounding is part of the result) and reduced
-// mod 2 pi before sincos (phases reach ~1e7 rad).  FP64 throughout.
+// per trajectory segment); a thread finds its samples' segments by bisection over
+// the segments' first samples.
+//   * Amplitudes.  The three Bessel combinations of a harmonic depend on e alone,
+//     and e hardly moves over the few hundred samples of a CTA: they are computed
+//     at 6, 8 or 12 Chebyshev nodes of the CTA's own range of e (the fewest whose
+//     interpolation error stays below 1e-17) and evaluated as polynomials there.
+//     At a node the five Bessel values of a harmonic come from one backward
+//     (Miller) recurrence normalised by J_0 + 2 sum J_2k = 1.  Where e moves too
+//     far for 12 nodes, every sample runs the recurrence.
+//   * Phases.  e^{i n Phi} by a running product of e^{i Phi}; the reference rounds
+//     n Phi (+ Doppler), at phases of ~1e7 rad, and that rounding is part of the
+//     result: its exact error eps (|eps| < 4e-9) comes from error-free
+//     transformations and enters as the factor 1 - i eps.
+//   * The three sums over harmonics leave the orientation, the polarisation
+//     rotation and the response to be applied once per sample.
+// FP64 throughout.
 #include <cuda_runtime.h>
 
 #include <cmath>
 #include <vector>
 
+#include "few_common.cuh"
 #include "few_internal.h"
 
 namespace few {
@@ -34,21 +45,6 @@ constexpr double kMTSUN = 4.9254909491978065e-06;      // solar mass in s (globa
 constexpr double kGPCINSEC = 1.02927125054339e+17;     // Gpc in s (global.h:26)
 constexpr double kAUsec = 499.00478383615643;          // AU in s (global.h:27)
 constexpr double kYRSID = 31558149.763545595;          // sidereal year in s (global.h:23)
-
-// e^{i ph} for large ph: Cody & Waite reduction mod 2 pi (three-part split,
-// k*C1 and k*C2 exact for |k| < 2^21), then sincos on |r| <= pi.
-__device__ __forceinline__ void sincos_big(double ph, double *s, double *c) {
-    const double kInv2Pi = 0.15915494309189535;
-    const double kC1 = 0x1.921fb54400000p+2, kC2 = 0x1.0b4611a600000p-32, kC3 = 0x1.3198a2e037073p-67;
-    double r = ph;
-    double kq = rint(ph * kInv2Pi);
-    if (fabs(kq) < 2097152.0) {
-        r = __fma_rn(-kq, kC1, ph);
-        r = __fma_rn(-kq, kC2, r);
-        r = __fma_rn(-kq, kC3, r);
-    }
-    sincos(r, s, c);
-}
 
 // J_{n-2}(x) .. J_{n+2}(x) into J[0..4] for n >= 1, x >= 0 (J_{-1} = -J_1), by
 // Miller's backward recurrence b_{k-1} = (2k/x) b_k - b_{k+1} from a start
@@ -202,22 +198,149 @@ __device__ __forceinline__ void cross3(const double *u, const double *v, double 
     w[2] = u[0] * v[1] - u[1] * v[0];
 }
 
-__global__ void __launch_bounds__(128) k_aak(AakArgs A) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i0 = A.first[0], i1 = A.first[A.nseg];
-    if (i < i0 || i >= i1) return;
-    // segment j with first[j] <= i < first[j+1]
-    int lo = 0, hi = A.nseg - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (A.first[mid] <= i) lo = mid; else hi = mid - 1;
+// ---- Chebyshev interpolation on Q nodes ------------------------------------------
+// node[j] = cos((j + 1/2) pi / Q); v[k][j]: the coefficient of u^k of the interpolant
+// is sum_j v[k][j] f(node_j) (the discrete Chebyshev coefficients, then T_m by
+// powers of u).
+constexpr double const_cos(double x) {  // Taylor, 0 <= x <= pi
+    const bool flip = x > 1.5707963267948966;
+    const double r = flip ? kPi - x : x;
+    double term = 1.0, sum = 1.0;
+    for (int k = 1; k < 16; ++k) {
+        term *= -r * r / ((2.0 * k - 1.0) * (2.0 * k));
+        sum += term;
     }
-    const int j = lo;
-    double c[5][8];
+    return flip ? -sum : sum;
+}
+
+constexpr int kMaxNodes = 12;
+
+struct Cheb {
+    double node[kMaxNodes];
+    double v[kMaxNodes][kMaxNodes];
+};
+
+constexpr Cheb make_cheb(int Q) {
+    Cheb t{};
+    double T[kMaxNodes][kMaxNodes] = {};  // T_m by powers
+    T[0][0] = 1.0;
+    T[1][1] = 1.0;
+    for (int m = 2; m < Q; ++m)
+        for (int k = 0; k < Q; ++k) T[m][k] = (k > 0 ? 2.0 * T[m - 1][k - 1] : 0.0) - T[m - 2][k];
+    for (int j = 0; j < Q; ++j) {
+        t.node[j] = const_cos((j + 0.5) * kPi / Q);
+        double c[kMaxNodes] = {};  // T_m(node_j)
+        c[0] = 1.0;
+        c[1] = t.node[j];
+        for (int m = 2; m < Q; ++m) c[m] = 2.0 * t.node[j] * c[m - 1] - c[m - 2];
+        for (int k = 0; k < Q; ++k) {
+            double sum = 0.0;
+            for (int m = 0; m < Q; ++m) sum += (m == 0 ? 1.0 : 2.0) / Q * c[m] * T[m][k];
+            t.v[k][j] = sum;
+        }
+    }
+    return t;
+}
+
+__constant__ Cheb c_cheb[3] = {make_cheb(6), make_cheb(8), make_cheb(12)};
+
+constexpr int kThreads = 128;
+constexpr int kHarm = 24;  // harmonics whose polynomials a CTA holds at a time (even: they come in pairs)
+
+// Largest n * (half width of the e range) for Q nodes: the interpolant of a
+// function whose Q-th derivative is at most n^Q errs by at most
+// (n delta)^Q / (2^(Q-1) Q!), kept below 1e-17.
+__device__ __forceinline__ int node_set(double nd) { return nd <= 7.8e-3 ? 0 : (nd <= 0.052 ? 1 : (nd <= 0.38 ? 2 : 3)); }
+
+// The three combinations of harmonic n's Bessel values J_{n-2..n+2}(n e).
+__device__ __forceinline__ void combine(int n, double e, const double J[5], double f[3]) {
+    f[0] = -n * (J[0] - 2. * e * J[1] + 2. / n * J[2] + 2. * e * J[3] - J[4]);
+    f[1] = -n * (J[0] - 2. * J[2] + J[4]);
+    f[2] = 2. * J[2];
+}
+
+// Per-launch angles, once per CTA (one sine and cosine a lane).
+struct Sky {
+    double sinqS, cosqS, sinqK, cosqK, sinPS, cosPS, sinPK, cosPK, sindP, cosdP;  // dP = phiK - phiS
+};
+
+// Sums of one group of harmonics [n0, n0 + count) for the thread's P samples, with
+// Q coefficients per function in co[(harmonic * 3 + function) * kMaxNodes + k].
+template <int P, bool MICH>
+struct Harmonics {
+    double u[P], Phi[P];                // position in the CTA's e range, Phi_r
+    double2 E[P], Z[P];                 // e^{i Phi} (and the Doppler's share), its running power
+    double Sa[P], Sb[P], Sc[P];
+    double nu[P], gd[P], W[P];          // Doppler of harmonic n: W (n nu + gd)  (MICH)
+    bool large;                         // phases past the first-order rounding factor: sincos for each
+
+    // e^{i nPhi} of harmonic n for sample q, nPhi rounded as the reference rounds it
+    __device__ __forceinline__ void phasor(int n, int q, const AakArgs &A, const Sky &K, const double *cosorb,
+                                           double &cn, double &sn) const {
+        const double dn = (double)n;
+        double nPhi, eps;
+        if (MICH) {
+            const double fn = fma(dn, nu[q], gd[q]);
+            const double D = 2. * kPi * fn * kAUsec * K.sinqS * cosorb[q];
+            nPhi = fma(dn, Phi[q], D);
+            const double p = rmul(dn, Phi[q]), pe = fma(dn, Phi[q], -p);
+            const double t = radd(p, D);
+            eps = (rsub(t, nPhi) + two_sum_err(p, D, t)) + pe;
+        } else {
+            nPhi = rmul(dn, Phi[q]);
+            eps = fma(dn, Phi[q], -nPhi);
+        }
+        if (large) {
+            sincos_phase(nPhi, &sn, &cn);
+        } else {
+            cn = fma(Z[q].y, eps, Z[q].x);
+            sn = fma(-Z[q].x, eps, Z[q].y);
+        }
+    }
+
+    template <int Q>
+    __device__ __forceinline__ void table(int n0, int count, const double *co, const AakArgs &A, const Sky &K,
+                                          const double *cosorb) {
+        for (int h = 0; h < count; ++h) {
+            const double *c = co + h * 3 * kMaxNodes;
+            double f[3][P];
 #pragma unroll
-    for (int q = 0; q < 5; ++q)
+            for (int w = 0; w < 3; ++w) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) c[q][k] = A.coef[((long long)k * A.cstride + j) * 6 + (q + 1)];
+                for (int q = 0; q < P; ++q) f[w][q] = c[w * kMaxNodes + Q - 1];
+#pragma unroll
+                for (int k = Q - 2; k >= 0; --k) {
+                    const double ck = c[w * kMaxNodes + k];
+#pragma unroll
+                    for (int q = 0; q < P; ++q) f[w][q] = fma(f[w][q], u[q], ck);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < P; ++q) {
+                double cn, sn;
+                phasor(n0 + h, q, A, K, cosorb, cn, sn);
+                Sa[q] = fma(f[0][q], cn, Sa[q]);
+                Sb[q] = fma(f[1][q], sn, Sb[q]);
+                Sc[q] = fma(f[2][q], cn, Sc[q]);
+                Z[q] = cmul(Z[q], E[q]);
+            }
+        }
+    }
+};
+
+// Bound by FP64 latency and issue at 16 warps per SM.  One year at dt = 10 s, 18
+// harmonics: 0.39 ms (2.02 ms with the nine recurrences, a sincos per harmonic and
+// the geometry's angles per sample), with the response 0.59 ms (2.17 ms).  A few
+// thousand samples of 24 harmonics: 16 us (41 us).
+template <int P, bool MICH>
+__global__ void __launch_bounds__(kThreads, 4) k_aak(AakArgs A) {
+    __shared__ Sky K;
+    __shared__ double s_co[kHarm * 3 * kMaxNodes];
+    __shared__ double s_min[kThreads / 32], s_max[kThreads / 32];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int i0 = A.first[0], i1 = A.first[A.nseg];
+    const int chunk = i0 + (int)blockIdx.x * (kThreads * P);
+    if (chunk >= i1) return;
 
     double qS = A.qS, qK = A.qK;
     const double fill = 1e-6;
@@ -225,132 +348,260 @@ __global__ void __launch_bounds__(128) k_aak(AakArgs A) {
     if (qK < fill) qK = fill;
     if (qS > kPi - fill) qS = kPi - fill;
     if (qK > kPi - fill) qK = kPi - fill;
-    double sinqS, cosqS, sinqK, cosqK, sinphiK, cosphiK;
-    sincos(qS, &sinqS, &cosqS);
-    sincos(qK, &sinqK, &cosqK);
-    sincos(A.phiK, &sinphiK, &cosphiK);
+    if (tid < 5) {
+        const double ang = tid == 0 ? qS : tid == 1 ? qK : tid == 2 ? A.phiS : tid == 3 ? A.phiK : A.phiK - A.phiS;
+        double sn, cs;
+        sincos(ang, &sn, &cs);
+        double *d = &K.sinqS + 2 * tid;
+        d[0] = sn;
+        d[1] = cs;
+    }
+
+    // segment of each sample: the last j with first[j] <= i
+    int seg[P];
+    double sa[P], e[P];
+    double emin = INFINITY, emax = -INFINITY;
+#pragma unroll
+    for (int q = 0; q < P; ++q) {
+        const int i = min(chunk + tid + q * kThreads, i1 - 1);
+        int lo = 0, hi = A.nseg - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (A.first[mid] <= i) lo = mid; else hi = mid - 1;
+        }
+        seg[q] = lo;
+        const double h = A.t[lo + 1] - A.t[lo];
+        sa[q] = (A.dt * i - A.t[lo]) / h;
+        double c[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) c[k] = A.coef[((long long)k * A.cstride + lo) * 6 + 1];
+        e[q] = nested(c, sa[q], 1.0 - sa[q]);
+        emin = fmin(emin, e[q]);
+        emax = fmax(emax, e[q]);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        emin = fmin(emin, __shfl_xor_sync(0xffffffffu, emin, off));
+        emax = fmax(emax, __shfl_xor_sync(0xffffffffu, emax, off));
+    }
+    if (lane == 0) {
+        s_min[tid >> 5] = emin;
+        s_max[tid >> 5] = emax;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) {
+        emin = fmin(emin, s_min[w]);
+        emax = fmax(emax, s_max[w]);
+    }
+    const double ec = 0.5 * (emin + emax), delta = fmax(0.5 * (emax - emin), 1e-15);
+
+    Harmonics<P, MICH> H;
+    double cosorb[P];
+    H.large = false;
+#pragma unroll
+    for (int q = 0; q < P; ++q) {
+        const int j = seg[q];
+        const double s = sa[q], s1 = 1.0 - s;
+        double c[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) c[k] = A.coef[((long long)k * A.cstride + j) * 6 + 5];
+        H.Phi[q] = nested(c, s, s1);
+        H.large = H.large || !(fabs(H.Phi[q]) * A.nmodes < 3e7);
+        H.u[q] = (e[q] - ec) / delta;
+        double sn, cs;
+        sincos_phase(H.Phi[q], &sn, &cs);
+        H.E[q] = make_double2(cs, sn);
+        H.Z[q] = H.E[q];
+        H.Sa[q] = H.Sb[q] = H.Sc[q] = 0.0;
+        cosorb[q] = 0.0;
+        if (MICH) {
+            const double h = A.t[j + 1] - A.t[j];
+            const double Om_r = nested_ds(c, s, h);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) c[k] = A.coef[((long long)k * A.cstride + j) * 6 + 4];
+            const double Om_theta = nested_ds(c, s, h);
+            H.nu[q] = Om_r / (2. * kPi);
+            H.gd[q] = (Om_theta - Om_r) / kPi;
+            const int i = min(chunk + tid + q * kThreads, i1 - 1);
+            cosorb[q] = cos(2. * kPi * (A.dt * i) / kYRSID - A.phiS);
+            H.W[q] = 2. * kPi * kAUsec * K.sinqS * cosorb[q];
+            sincos(H.W[q] * H.nu[q], &sn, &cs);
+            H.E[q] = cmul(H.E[q], make_double2(cs, sn));
+            sincos(H.W[q] * H.gd[q], &sn, &cs);
+            H.Z[q] = cmul(H.E[q], make_double2(cs, sn));
+            H.large = H.large || !(fabs(H.W[q] * H.nu[q]) * A.nmodes < 1e6);
+        }
+    }
+
+    for (int n0 = 1; n0 <= A.nmodes; n0 += kHarm) {
+        const int count = min(kHarm, A.nmodes + 1 - n0);
+        const int set = node_set((n0 + count - 1) * delta);
+        if (set < 3) {
+            const int Q = set == 0 ? 6 : (set == 1 ? 8 : 12);
+            const Cheb &T = c_cheb[set];
+            __syncthreads();  // the previous group's coefficients have been read
+            const int pairs = (count + 1) / 2;
+            for (int w = tid; w < pairs * Q; w += kThreads) {
+                const int pr = w / Q, j = w - pr * Q, n = n0 + 2 * pr;
+                const double en = fma(delta, T.node[j], ec);
+                double Ja[5], Jb[5], f[3];
+                bessel_band2(n, n * en, (n + 1) * en, Ja, Jb);
+                combine(n, en, Ja, f);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) s_co[(2 * pr * 3 + q) * kMaxNodes + j] = f[q];
+                combine(n + 1, en, Jb, f);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) s_co[((2 * pr + 1) * 3 + q) * kMaxNodes + j] = f[q];
+            }
+            __syncthreads();
+            // values at the nodes -> coefficients of the powers of u, in place
+            for (int w = tid; w < count * 3; w += kThreads) {
+                double *c = s_co + w * kMaxNodes;
+                double f[kMaxNodes];
+#pragma unroll
+                for (int j = 0; j < kMaxNodes; ++j) f[j] = j < Q ? c[j] : 0.0;
+                for (int k = 0; k < Q; ++k) {
+                    double sum = 0.0;
+#pragma unroll
+                    for (int j = 0; j < kMaxNodes; ++j) sum = fma(T.v[k][j], f[j], sum);
+                    c[k] = sum;
+                }
+            }
+            __syncthreads();
+            if (set == 0) H.template table<6>(n0, count, s_co, A, K, cosorb);
+            else if (set == 1) H.template table<8>(n0, count, s_co, A, K, cosorb);
+            else H.template table<12>(n0, count, s_co, A, K, cosorb);
+        } else {
+#pragma unroll
+            for (int q = 0; q < P; ++q) {
+                double Ja[5], Jb[5], f[3];
+                for (int h = 0; h < count; ++h) {
+                    const int n = n0 + h;
+                    const bool odd = (n & 1) != 0;
+                    if (odd) bessel_band2(n, n * e[q], (n + 1) * e[q], Ja, Jb);  // the last n + 1 may go unused
+                    double J[5];
+#pragma unroll
+                    for (int k = 0; k < 5; ++k) J[k] = odd ? Ja[k] : Jb[k];
+                    combine(n, e[q], J, f);
+                    double cn, sn;
+                    H.phasor(n, q, A, K, cosorb, cn, sn);
+                    H.Sa[q] = fma(f[0], cn, H.Sa[q]);
+                    H.Sb[q] = fma(f[1], sn, H.Sb[q]);
+                    H.Sc[q] = fma(f[2], cn, H.Sc[q]);
+                    H.Z[q] = cmul(H.Z[q], H.E[q]);
+                }
+            }
+        }
+    }
+
     const double halfsqrt3 = sqrt(3.) / 2.;
     const double zeta = A.mu * kMTSUN / A.dist / kGPCINSEC;
+    const double nv[3] = {K.sinqS * K.cosPS, K.sinqS * K.sinPS, K.cosqS};
+    const double Sv[3] = {K.sinqK * K.cosPK, K.sinqK * K.sinPK, K.cosqK};
+    double nxS[3];
+    cross3(nv, Sv, nxS);
+    const double nS = sqrt(nxS[0] * nxS[0] + nxS[1] * nxS[1] + nxS[2] * nxS[2]);
+    const double Sdotn = K.cosqK * K.cosqS + K.sinqK * K.sinqS * K.cosdP;
+#pragma unroll
+    for (int q = 0; q < P; ++q) {
+        const int i = chunk + tid + q * kThreads;
+        if (i >= i1) continue;
+        const int j = seg[q];
+        const double s = sa[q], s1 = 1.0 - s;
+        double c[3][8];  // Y, Phi_phi, Phi_theta
+#pragma unroll
+        for (int w = 0; w < 3; ++w)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) c[w][k] = A.coef[((long long)k * A.cstride + j) * 6 + w + 2];
+        const double h = A.t[j + 1] - A.t[j];
+        const double Y = nested(c[0], s, s1), Phi_phi = nested(c[1], s, s1), Phi_theta = nested(c[2], s, s1);
+        const double Om_phi = nested_ds(c[1], s, h);
+        const double gim = Phi_theta - H.Phi[q], alp = Phi_phi - Phi_theta;
+        // lam = acos(Y): its cosine is Y, its sine the root below
+        const double coslam = Y, sinlam = sqrt((1.0 - Y) * (1.0 + Y));
+        double sinalp, cosalp;
+        sincos_phase(alp, &sinalp, &cosalp);
+        const double Lv[3] = {coslam * K.sinqK * K.cosPK + sinlam * (sinalp * K.sinPK - cosalp * K.cosqK * K.cosPK),
+                              coslam * K.sinqK * K.sinPK - sinlam * (sinalp * K.cosPK + cosalp * K.cosqK * K.sinPK),
+                              coslam * K.cosqK + sinlam * cosalp * K.sinqK};
+        // cos q_L cos q_S + sin q_L sin q_S cos(phi_L - phi_S), sin q_L from cos q_L as the
+        // reference forms it (it loses digits near the poles, and they show in the result)
+        const double horiz = Lv[0] * Lv[0] + Lv[1] * Lv[1];
+        const double cosL = horiz > 0.0 ? (Lv[0] * K.cosPS + Lv[1] * K.sinPS) / sqrt(horiz) : K.cosPS;
+        const double Ldotn = Lv[2] * K.cosqS + sqrt(1. - Lv[2] * Lv[2]) * K.sinqS * cosL;
+        const double Ldotn2 = Ldotn * Ldotn;
+        double beta = 0.0;
+        if (!(A.S == 0.0 || fabs(Y) == 1.0)) {  // lam within 1e-10 of 0 or pi only when |Y| = 1
+            const double up = -Sdotn + coslam * Ldotn;
+            const double down =
+                K.sinqS * K.sindP * sinlam * cosalp + (K.cosqK * Sdotn - K.cosqS) / K.sinqK * sinlam * sinalp;
+            beta = atan2(up, down);
+        }
+        double sin2gam, cos2gam;
+        sincos_phase(2. * (gim + beta), &sin2gam, &cos2gam);
 
-    const double t = A.dt * i;
-    const double h = A.t[j + 1] - A.t[j];
-    const double s = (t - A.t[j]) / h, s1 = 1.0 - s;
-    const double e = nested(c[0], s, s1), Y = nested(c[1], s, s1);
-    const double Phi_phi = nested(c[2], s, s1), Phi_theta = nested(c[3], s, s1), Phi_r = nested(c[4], s, s1);
-    const double Om_phi = nested_ds(c[2], s, h), Om_theta = nested_ds(c[3], s, h), Om_r = nested_ds(c[4], s, h);
+        double FpI = 1.0, FcI = 0.0, FpII = 0.0, FcII = 1.0;
+        if (MICH) {
+            const double orb = 2. * kPi * (A.dt * i) / kYRSID;
+            double sorb, corb;
+            sincos(orb, &sorb, &corb);
+            const double sinorb = sorb * K.cosPS - corb * K.sinPS;  // of orb - phiS
+            const double cosq = .5 * K.cosqS - halfsqrt3 * K.sinqS * cosorb[q];
+            // phiw = orb + atan2(wy, wx); twice the angles enter, as (x + iy)^2 / |x + iy|^2
+            const double wy = halfsqrt3 * K.cosqS + .5 * K.sinqS * cosorb[q], wx = K.sinqS * sinorb;
+            const double psiup = .5 * K.cosqK - halfsqrt3 * K.sinqK * (corb * K.cosPK + sorb * K.sinPK) -
+                                 cosq * (K.cosqK * K.cosqS + K.sinqK * K.sinqS * K.cosdP);
+            const double psidown = .5 * K.sinqK * K.sinqS * K.sindP -
+                                   halfsqrt3 * corb * (K.cosqK * K.sinqS * K.sinPS - K.cosqS * K.sinqK * K.sinPK) -
+                                   halfsqrt3 * sorb * (K.cosqS * K.sinqK * K.cosPK - K.cosqK * K.sinqS * K.cosPS);
+            const double cosq1 = .5 * (1. + cosq * cosq);
+            const double zx = wx * corb - wy * sorb, zy = wx * sorb + wy * corb;
+            const double zr = zx * zx + zy * zy, pr = psiup * psiup + psidown * psidown;
+            const double s2phi = zr > 0.0 ? 2. * zx * zy / zr : 0.0, c2phi = zr > 0.0 ? (zx - zy) * (zx + zy) / zr : 1.0;
+            const double s2psi = pr > 0.0 ? 2. * psiup * psidown / pr : 0.0;
+            const double c2psi = pr > 0.0 ? (psidown - psiup) * (psidown + psiup) / pr : 1.0;
+            FpI = halfsqrt3 * (cosq1 * c2phi * c2psi - cosq * s2phi * s2psi);
+            FcI = halfsqrt3 * (cosq1 * c2phi * s2psi + cosq * s2phi * c2psi);
+            FpII = halfsqrt3 * (cosq1 * s2phi * c2psi + cosq * c2phi * s2psi);
+            FcII = halfsqrt3 * (cosq1 * s2phi * s2psi - cosq * c2phi * c2psi);
+        }
+        const double root = cbrt(fabs(Om_phi) * A.M * kMTSUN);
+        const double Amp = root * root * zeta;
 
-    const double Phi = Phi_r, gim = Phi_theta - Phi_r, alp = Phi_phi - Phi_theta;
-    const double nu = Om_r / (2. * kPi), gimdot = Om_theta - Om_r;
-    const double lam = acos(Y);
-    double sinlam, coslam, sinalp, cosalp;
-    sincos(lam, &sinlam, &coslam);
-    sincos_big(alp, &sinalp, &cosalp);
-    const double cosqL = cosqK * coslam + sinqK * sinlam * cosalp;
-    const double sinqL = sqrt(1. - cosqL * cosqL);
-    const double phiLup = sinqK * sinphiK * coslam - cosphiK * sinlam * sinalp - cosqK * sinphiK * sinlam * cosalp;
-    const double phiLdown = sinqK * cosphiK * coslam + sinphiK * sinlam * sinalp - cosqK * cosphiK * sinlam * cosalp;
-    const double phiL = atan2(phiLup, phiLdown);
-    const double Ldotn = cosqL * cosqS + sinqL * sinqS * cos(phiL - A.phiS);
-    const double Ldotn2 = Ldotn * Ldotn;
-    const double Sdotn = cosqK * cosqS + sinqK * sinqS * cos(A.phiK - A.phiS);
-    double beta = 0.0;
-    if (!(A.S == 0.0 || lam < 1e-10 || lam > (kPi - 1e-10))) {
-        const double up = -Sdotn + coslam * Ldotn;
-        const double down = sinqS * sin(A.phiK - A.phiS) * sinlam * cosalp + (cosqK * Sdotn - cosqS) / sinqK * sinlam * sinalp;
-        beta = atan2(up, down);
-    }
-    double sin2gam, cos2gam;
-    sincos_big(2. * (gim + beta), &sin2gam, &cos2gam);
-
-    double FpI = 1.0, FcI = 0.0, FpII = 0.0, FcII = 1.0, cosorb = 0.0;
-    if (A.mich) {
-        const double orb = 2. * kPi * t / kYRSID;
-        double sinorb;
-        sincos(orb - A.phiS, &sinorb, &cosorb);
-        const double cosq = .5 * cosqS - halfsqrt3 * sinqS * cosorb;
-        const double phiw = orb + atan2(halfsqrt3 * cosqS + .5 * sinqS * cosorb, sinqS * sinorb);
-        const double psiup = .5 * cosqK - halfsqrt3 * sinqK * cos(orb - A.phiK) -
-                             cosq * (cosqK * cosqS + sinqK * sinqS * cos(A.phiK - A.phiS));
-        const double psidown = .5 * sinqK * sinqS * sin(A.phiK - A.phiS) -
-                               halfsqrt3 * cos(orb) * (cosqK * sinqS * sin(A.phiS) - cosqS * sinqK * sin(A.phiK)) -
-                               halfsqrt3 * sin(orb) * (cosqS * sinqK * cos(A.phiK) - cosqK * sinqS * cos(A.phiS));
-        const double psi = atan2(psiup, psidown);
-        const double cosq1 = .5 * (1. + cosq * cosq);
-        double s2phi, c2phi, s2psi, c2psi;
-        sincos(2. * phiw, &s2phi, &c2phi);
-        sincos(2. * psi, &s2psi, &c2psi);
-        FpI = cosq1 * c2phi * c2psi - cosq * s2phi * s2psi;
-        FcI = cosq1 * c2phi * s2psi + cosq * s2phi * c2psi;
-        FpII = cosq1 * s2phi * c2psi + cosq * c2phi * s2psi;
-        FcII = cosq1 * s2phi * s2psi - cosq * c2phi * c2psi;
-    }
-    const double Amp = pow(fabs(Om_phi) * A.M * kMTSUN, 2. / 3.) * zeta;
-
-    // polarisation rotation (gpuAAK.cu:141-177)
-    double rot0, rot1;
-    {
-        double sinS, cosS, sinPS, cosPS, sinK, cosK, sinPK, cosPK, sini, cosi;
-        sincos(qS, &sinS, &cosS);
-        sincos(A.phiS, &sinPS, &cosPS);
-        sincos(qK, &sinK, &cosK);
-        sincos(A.phiK, &sinPK, &cosPK);
-        sincos(lam, &sini, &cosi);
-        const double nv[3] = {sinS * cosPS, sinS * sinPS, cosS};
-        const double Sv[3] = {sinK * cosPK, sinK * sinPK, cosK};
-        const double Lv[3] = {cosi * sinK * cosPK + sini * (sinalp * sinPK - cosalp * cosK * cosPK),
-                              cosi * sinK * sinPK - sini * (sinalp * cosPK + cosalp * cosK * sinPK),
-                              cosi * cosK + sini * cosalp * sinK};
-        double nxL[3], nxS[3];
+        // polarisation rotation (gpuAAK.cu:141-177)
+        double nxL[3];
         cross3(nv, Lv, nxL);
-        cross3(nv, Sv, nxS);
-        double norm = sqrt(nxL[0] * nxL[0] + nxL[1] * nxL[1] + nxL[2] * nxL[2]) *
-                      sqrt(nxS[0] * nxS[0] + nxS[1] * nxS[1] + nxS[2] * nxS[2]);
+        double norm = sqrt(nxL[0] * nxL[0] + nxL[1] * nxL[1] + nxL[2] * nxL[2]) * nS;
         if (norm < 1e-6) norm = 1e-6;
         const double cosrot = (nxL[0] * nxS[0] + nxL[1] * nxS[1] + nxL[2] * nxS[2]) / norm;
-        double sinrot = Lv[0] * nxS[0] + Lv[1] * nxS[1] + Lv[2] * nxS[2];
-        sinrot -= Sv[0] * nxL[0] + Sv[1] * nxL[1] + Sv[2] * nxL[2];
-        sinrot /= norm;
-        rot0 = 2. * cosrot * cosrot - 1.;
-        rot1 = cosrot * sinrot;
-    }
-    const double rot2 = -rot1, rot3 = rot0;
-    const double sqrt1me2 = sqrt(1 - e * e);
+        const double sinrot = (Lv[0] * nxS[0] + Lv[1] * nxS[1] + Lv[2] * nxS[2] -
+                               (Sv[0] * nxL[0] + Sv[1] * nxL[1] + Sv[2] * nxL[2])) /
+                              norm;
+        const double rot0 = 2. * cosrot * cosrot - 1., rot1 = cosrot * sinrot;
 
-    double hI = 0.0, hII = 0.0;
-    double Ja[5], Jb[5];  // Bessel bands of the odd harmonic n and of n + 1
-    for (int n = 1; n <= A.nmodes; ++n) {
-        double nPhi;
-        if (A.mich) {
-            const double fn = n * nu + gimdot / kPi;
-            const double Doppler = 2. * kPi * fn * kAUsec * sinqS * cosorb;
-            nPhi = n * Phi + Doppler;
-        } else {
-            nPhi = n * Phi;
-        }
-        // Bessel values two harmonics at a time (odd n computes n and n + 1)
-        const bool odd = (n & 1) != 0;
-        if (odd) bessel_band2(n, n * e, (n + 1) * e, Ja, Jb);  // the last n + 1 may go unused
-        double J[5];
-#pragma unroll
-        for (int q = 0; q < 5; ++q) J[q] = odd ? Ja[q] : Jb[q];
-        double sn, cn;
-        sincos_big(nPhi, &sn, &cn);
-        const double a = -n * Amp * (J[0] - 2. * e * J[1] + 2. / n * J[2] + 2. * e * J[3] - J[4]) * cn;
-        const double b = -n * Amp * sqrt1me2 * (J[0] - 2. * J[2] + J[4]) * sn;
-        const double cc = 2. * Amp * J[2] * cn;
+        const double a = Amp * H.Sa[q], b = Amp * sqrt(1 - e[q] * e[q]) * H.Sb[q], cc = Amp * H.Sc[q];
         const double Ap0 = -(1. + Ldotn2) * (a * cos2gam - b * sin2gam) + cc * (1 - Ldotn2);
         const double Ac0 = 2. * Ldotn * (b * cos2gam + a * sin2gam);
         const double Ap = Ap0 * rot0 + Ac0 * rot1;
-        const double Ac = Ap0 * rot2 + Ac0 * rot3;
-        if (A.mich) {
-            hI += halfsqrt3 * (FpI * Ap + FcI * Ac);
-            hII += halfsqrt3 * (FpII * Ap + FcII * Ac);
-        } else {
-            hI += FpI * Ap + FcI * Ac;
-            hII += FpII * Ap + FcII * Ac;
-        }
+        const double Ac = Ac0 * rot0 - Ap0 * rot1;
+        A.wf[i] = make_double2(FpI * Ap + FcI * Ac, -(FpII * Ap + FcII * Ac));
     }
-    A.wf[i] = make_double2(hI, -hII);
+}
+
+// Four samples a thread share each coefficient read, two with the response (whose
+// state for four spills: 0.60 against 0.59 ms at one year, 80 against 60 us at
+// 310,000 samples); one when more would leave SMs without a CTA.  Four CTAs per
+// SM: 0.39 ms plain at one year, 0.42 and 0.51 at three and two.
+int launch_aak(const AakArgs &A, int total, cudaStream_t st) {
+    const int per = total < 148 * 2 * 4 * kThreads ? 1 : (A.mich ? 2 : 4);
+    const int ctas = (total + per * kThreads - 1) / (per * kThreads);
+    if (per == 4) k_aak<4, false><<<ctas, kThreads, 0, st>>>(A);
+    else if (per == 2) k_aak<2, true><<<ctas, kThreads, 0, st>>>(A);
+    else if (A.mich) k_aak<1, true><<<ctas, kThreads, 0, st>>>(A);
+    else k_aak<1, false><<<ctas, kThreads, 0, st>>>(A);
+    FEW_LAUNCH_CHECK("k_aak");
+    return FEW_OK;
 }
 
 }  // namespace aak
@@ -401,9 +652,7 @@ extern "C" FEW_API int few_aak_sum(void *waveform, const double *coef, int cstri
     A.mich = mich;
     A.M = M_phys; A.S = S_phys; A.mu = mu; A.qS = qS; A.phiS = phiS; A.qK = qK; A.phiK = phiK; A.dist = dist;
     A.dt = delta_t;
-    few::aak::k_aak<<<(total + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(A);
-    FEW_LAUNCH_CHECK("k_aak");
-    return FEW_OK;
+    return few::aak::launch_aak(A, total, static_cast<cudaStream_t>(stream));
 }
 
 // Drop-in for get_waveform of gpuAAK.hh:6-10 (AAKSummation's kernel call,
@@ -447,10 +696,7 @@ extern "C" FEW_API int few_aak_waveform(void *waveform, const double *interp_arr
         A.mich = mich;
         A.M = M_phys; A.S = S_phys; A.mu = mu; A.qS = qS; A.phiS = phiS; A.qK = qK; A.phiK = phiK; A.dist = dist;
         A.dt = delta_t;
-        const int total = first.back();
-        few::aak::k_aak<<<(total + 127) / 128, 128, 0, st>>>(A);
-        cudaError_t e2 = cudaGetLastError();
-        if (e2 != cudaSuccess) status = few::fail(FEW_ERR_CUDA, "launch of k_aak failed: %s", cudaGetErrorString(e2));
+        status = few::aak::launch_aak(A, first.back(), st);
     }
     // the host vector must outlive the copy
     cudaError_t e3 = cudaStreamSynchronize(st);
