@@ -85,6 +85,8 @@ SIGNATURES = {
     "few_fd_finalize": [_vp, _c_int, _c_int, _c_int, _vp, _vp],
     "few_ylm": [_vp, _vp, _c_int, _c_int, _c_dbl, _c_dbl, _vp, _vp, _vp],
     "few_mode_snr2": [_vp, _c_int, _c_int, _vp, _vp, _vp, _vp, _vp, _vp],
+    "few_mode_select_max": [],
+    "few_mode_select": [_vp, _c_int, _c_dbl, _c_int, _c_int, _vp, _vp, _vp, _vp, _vp, _vp],
     "few_mode_keep": [_vp, _c_int, _c_dbl, _vp, _vp],
     "few_direct_sum": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _c_int, _c_int, _vp, _vp],
     "few_aak_sum": [_vp, _vp, _c_int, _vp, _vp, _c_int, _c_int, _c_dbl, _c_dbl, _c_dbl, _c_dbl, _c_dbl, _c_dbl,

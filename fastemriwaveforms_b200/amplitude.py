@@ -18,7 +18,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .summation import _device, _ptr, _stream
+from .summation import _device, _ptr, _stream, _upload
 
 
 def _dev_f64(x, dev) -> torch.Tensor:
@@ -61,8 +61,8 @@ class AmpInterp2D:
         u_h = u.detach().cpu().numpy() if isinstance(u, torch.Tensor) else np.asarray(u, dtype=np.float64)
         if w_h.shape != u_h.shape:
             w_h, u_h = np.broadcast_arrays(w_h, u_h)
-        w_d = _dev_f64(np.ravel(w_h), dev)
-        u_d = _dev_f64(np.ravel(u_h), dev)
+        w_d = _upload(np.ravel(w_h).astype(np.float64, copy=False), dev)
+        u_d = _upload(np.ravel(u_h).astype(np.float64, copy=False), dev)
         m = int(w_d.shape[0])
         if mode_indexes is None:
             idx = None
@@ -73,7 +73,7 @@ class AmpInterp2D:
             nmodes = int(idx.shape[0])
             if nmodes and (int(idx.min()) < 0 or int(idx.max()) >= self.num_teuk_modes):
                 raise ValueError("mode_indexes out of range.")
-        out = torch.zeros((m, nmodes), dtype=torch.complex128, device=dev)
+        out = torch.empty((m, nmodes), dtype=torch.complex128, device=dev)  # every element is written
         if m == 0 or nmodes == 0:
             return out
         tw, tu = self.knots

@@ -11,8 +11,10 @@ same outputs (teuk_modes, ylms, l, m, k, n).
 
 The threshold form runs on the device: ``k_mode_snr2`` (``csrc/modeselect.cu``)
 fuses the per-mode power |A Y|^2 (+ |conj(A) Y^-|^2 for m != 0), the optional
-sensitivity weights and the knot-interval sum; torch sorts the K estimates;
-``k_mode_keep`` applies the cumulative rule in sorted order.  ``GetYlms`` from
+sensitivity weights and the knot-interval sum; ``k_mode_rank`` and
+``k_mode_select`` sort the K estimates, apply the cumulative rule in that order and
+list the kept modes (``torch.sort`` and ``k_mode_keep`` for lists longer than they
+take); the host waits once, for the number of kept modes.  ``GetYlms`` from
 ``fastemriwaveforms_b200.ylm`` is the default harmonic generator.
 
 Deliberate difference: with ``include_minus_mkn=False`` outside the list form
@@ -27,8 +29,8 @@ import numpy as np
 import torch
 
 from . import _lib
-from .summation import _device, _ptr, _stream
-from .ylm import GetYlms
+from .summation import _device, _ptr, _stream, _to_device
+from .ylm import GetYlms, in_range, ylm_into
 
 logger = logging.getLogger("fastemriwaveforms_b200")
 
@@ -66,6 +68,11 @@ class ModeSelector:
         self.num_m_zero_up = int(self.m0mask.numel())
         self.num_m_1_up = int(self.m0mask.sum())
         self.num_m0 = self.num_m_zero_up - self.num_m_1_up
+        self._minus = self._minus_index()
+        # the (l, m) pairs of the harmonics as the kernel reads them, once they are known to be in its range
+        self._lm = None
+        if self.unique_l.shape == self.unique_m.shape and in_range(self.unique_l, self.unique_m):
+            self._lm = (self.unique_l.reshape(-1).to(torch.int32), self.unique_m.reshape(-1).to(torch.int32))
         self.sensitivity_fn = sensitivity_fn
         self.include_minus_mkn = include_minus_mkn
         self.mode_selection = mode_selection
@@ -105,7 +112,12 @@ class ModeSelector:
         return torch.as_tensor(arr, device=self.device)
 
     def _ylms_of_list(self, theta, phi):
-        y = self.ylm_generator(self.unique_l, self.unique_m, theta, phi)
+        if type(self.ylm_generator) is GetYlms and self._lm is not None and not self.ylm_generator.include_minus_m:
+            y = torch.empty(self._lm[0].numel(), dtype=torch.complex128, device=self.device)
+            if y.numel():
+                ylm_into(*self._lm, theta, phi, y)
+        else:
+            y = self.ylm_generator(self.unique_l, self.unique_m, theta, phi)
         return y[self.inverse_lm]
 
     def _minus_index(self):
@@ -163,7 +175,7 @@ class ModeSelector:
         teuk = _t(self.amplitude_generator(a, p, e, xI), torch.complex128, dev).contiguous()
         ylms = self._ylms_of_list(theta, phi).contiguous()
         N, K = teuk.shape
-        t_d = _t(t, torch.float64, dev).contiguous()
+        t_d = _to_device(t, torch.float64, dev)
         psd = None
         if self.sensitivity_fn is not None:
             f = online_mode_selection_args
@@ -172,19 +184,26 @@ class ModeSelector:
                                          self.n_arr.double()).abs()
             psd = _t(self.sensitivity_fn(freqs.flatten()), torch.float64, dev).reshape(freqs.shape).contiguous()
         snr2 = torch.empty(K, dtype=torch.float64, device=dev)
-        minus = self._minus_index()
         st = _stream(dev)
-        _lib.call("few_mode_snr2", _ptr(teuk), N, K, _ptr(ylms), _ptr(minus), _ptr(psd) if psd is not None else None,
-                  _ptr(t_d), _ptr(snr2), st)
-        vals, inds_sort = torch.sort(snr2, descending=True, stable=True)
-        keep_flag = torch.empty(K, dtype=torch.int32, device=dev)
-        _lib.call("few_mode_keep", _ptr(vals), K, float(mode_selection_threshold), _ptr(keep_flag), st)
-        keep_tmp = inds_sort[keep_flag.bool()]
-        keep_tmp = keep_tmp * (keep_tmp < self.num_m_zero_up) + (keep_tmp - self.num_m_1_up) * (
-            keep_tmp >= self.num_m_zero_up)
-        keep, inv = torch.unique(keep_tmp, sorted=True, return_inverse=True)
-        ylms_out = ylms[torch.cat([keep, idx_of_ylm_minus(keep)])]
-        out = (teuk[:, keep], ylms_out, self.l_arr[keep], self.m_arr[keep], self.k_arr[keep], self.n_arr[keep])
+        _lib.call("few_mode_snr2", _ptr(teuk), N, K, _ptr(ylms), _ptr(self._minus),
+                  _ptr(psd) if psd is not None else None, _ptr(t_d), _ptr(snr2), st)
+        if 1 <= K <= _lib.load().few_mode_select_max():
+            # kept modes, harmonics (two rows), ranks, scratch (two rows)
+            buf = torch.empty((6, K), dtype=torch.int64, device=dev)
+            count = torch.empty(1, dtype=torch.int32, device=dev)
+            _lib.call("few_mode_select", _ptr(snr2), K, float(mode_selection_threshold), self.num_m0, self.num_m_1_up,
+                      _ptr(buf[4]), _ptr(buf), _ptr(buf[1]), _ptr(buf[3]), _ptr(count), st)
+            c = int(count.item())
+            keep, ylm_idx, inv = buf[0, :c], buf[1:3].reshape(-1)[:2 * c], buf[3, :c]
+        else:
+            vals, inds_sort = torch.sort(snr2, descending=True, stable=True)
+            keep_flag = torch.empty(K, dtype=torch.int32, device=dev)
+            _lib.call("few_mode_keep", _ptr(vals), K, float(mode_selection_threshold), _ptr(keep_flag), st)
+            keep, inv = torch.unique(inds_sort[keep_flag.bool()], sorted=True, return_inverse=True)
+            ylm_idx = torch.cat([keep, idx_of_ylm_minus(keep)])
+        ylms_out = ylms[ylm_idx]
+        out = (teuk.index_select(1, keep), ylms_out, self.l_arr[keep], self.m_arr[keep], self.k_arr[keep],
+               self.n_arr[keep])
         if return_sort_inds:
             out += (inv,)
         return out

@@ -24,6 +24,11 @@ def ylm_into(l_d: torch.Tensor, m_d: torch.Tensor, theta: float, phi: float, out
               float(phi), _ptr(out), _ptr(status) if status is not None else None, _stream(out.device))
 
 
+def in_range(l: torch.Tensor, m: torch.Tensor) -> bool:
+    """Whether every (l, m) is one the kernel computes: 2 <= l <= 64, |m| <= l."""
+    return bool(((l >= 2) & (l <= 64) & (m.abs() <= l)).all())
+
+
 class GetYlms:
     """(-2) spin-weighted spherical harmonics Y_lm(theta, phi)."""
 

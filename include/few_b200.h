@@ -533,6 +533,20 @@ FEW_API int few_mode_snr2(const void *teuk, int N, int K, const void *ylms, cons
  * (1 - threshold)^2, with the cumulative sum taken in order. */
 FEW_API int few_mode_keep(const double *sorted_desc, int K, double threshold, int *keep, void *stream);
 
+/* Largest K of few_mode_select. */
+FEW_API int few_mode_select_max(void);
+
+/* From the estimates snr2 [device] (K,) to the kept modes (modeselector.py:
+ * 425-486): stable descending order (NaN first), the keep rule above, the kept
+ * modes in ascending order.  keep [device] (K,) int64: the kept modes; ylm_index
+ * [device] (2K,) int64: for the c kept modes their +m and then their -m
+ * harmonic's index (mode i: i for i < num_m0, else i + num_m_1_up); rank [device]
+ * (K,) int64: the position in keep of the i-th kept mode of the descending order;
+ * count [device] int: c.  Entries past c (2c for ylm_index) are not written.
+ * scratch [device]: 12 K bytes, 8-byte aligned. */
+FEW_API int few_mode_select(const double *snr2, int K, double threshold, int num_m0, int num_m_1_up, void *scratch,
+                            long long *keep, long long *ylm_index, long long *rank, int *count, void *stream);
+
 /* ------------------------------------------------------------------------ */
 /* Direct mode sum (DirectModeSum, src/few/summation/directmodesum.py)       */
 /* ------------------------------------------------------------------------ */
