@@ -1160,7 +1160,7 @@ def main():
     flops_per_key_sample = 30 if args.precision == "faithful" else 20
     sum_flops = float(keys) * T * flops_per_key_sample
     achieved = sum_flops / (stage["sum"] * 1e-3) / 1e12
-    spline_bytes = 40.0 * inp.num_knots * 2 * K
+    spline_bytes = 16.0 * inp.num_knots * 2 * K  # amplitude in, slope out
     # DRAM bytes of one launch at this workload from an ncu capture (dram__bytes_read.sum +
     # dram__bytes_write.sum); null for workloads not captured
     captured = args.workload == "plain_full" and args.precision == "faithful"
@@ -1171,13 +1171,11 @@ def main():
                 "peak_source": "measured in this run: few_probe_fp64_fma (FP64 FMA pipe)",
                 "algorithmic": f"{flops_per_key_sample} flop x {keys} keys x {T} samples per launch",
                 "launch_ms": stage["sum"]}
-    spline_roof = {"bound": "hbm", "kernel": "k_spline_build", "achieved": spline_bytes / (stage["spline"] * 1e-3) / 1e9,
+    spline_roof = {"bound": "hbm", "kernel": "k_spline_chunks", "achieved": spline_bytes / (stage["spline"] * 1e-3) / 1e9,
                    "peak": pk["hbm_gbs"], "unit": "GB/s",
                    "frac": spline_bytes / (stage["spline"] * 1e-3) / 1e9 / pk["hbm_gbs"],
-                   "peak_source": f"{pk_kind} hbm_gbs", "algorithmic": "40 B per (knot, series)",
-                   "traffic": ({"bytes_per_launch": 423.9e6,
-                                "source": "ncu capture of k_spline_build_factored (one-year workload)"}
-                               if args.workload == "plain_full" else None),
+                   "peak_source": f"{pk_kind} hbm_gbs", "algorithmic": "16 B per (knot, series)",
+                   "traffic": None,
                    "launch_ms": stage["spline"]}
 
     if rank != 0:

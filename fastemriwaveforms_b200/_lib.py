@@ -38,6 +38,11 @@ SIGNATURES = {
     "few_spline_eval": [_vp, _c_ll, _vp, _c_int, _c_int, _vp, _c_ll, _c_int, _c_int, _vp, _vp, _vp],
     "few_spline_factor": [_vp, _c_int, _vp],
     "few_spline_build_factored": [_vp, _vp, _c_ll, _c_ll, _c_int, _c_ll, _c_int, _c_int, _vp, _c_int, _vp],
+    "few_spline_overlap": [_vp, _c_int],
+    "few_spline_max_overlap": [],
+    "few_spline_build_chunked": [_vp, _c_int, _vp, _c_ll, _c_ll, _c_int, _c_ll, _c_int, _c_int, _vp, _c_int, _vp],
+    "few_spline_slopes": [_vp, _vp, _c_int, _c_int, _vp, _vp],
+    "few_fold_slopes": [_vp, _vp, _vp, _vp, _vp, _vp, _c_int, _c_int, _c_int, _c_int, _c_int, _vp, _vp],
     "few_fold_plan": [_vp, _vp, _vp, _c_int, _c_int, _c_int, _vp, _vp, _vp, _vp, _vp],
     "few_segment_plan": [_vp, _vp, _c_int, _c_int, _c_dbl, _c_int, _c_int, _vp, _vp, _vp, _vp],
     "few_fold_coeffs": [_vp, _vp, _vp, _vp, _c_int, _c_int, _c_int, _c_int, _c_int, _vp, _vp],

@@ -23,7 +23,7 @@ import numpy as np
 import torch
 
 from . import _lib, autotune
-from .summation import InterpolatedModeSum, _device, _ptr, _stream, _upload
+from .summation import InterpolatedModeSum, _device, _ptr, _stream, _upload, fold_amplitudes
 from .synthetic import output_length
 
 # Layout of few_wave_desc (include/few_b200.h): 8 pointers, 6 ints, 1 double.
@@ -116,7 +116,7 @@ class BatchedInterpolatedModeSum:
         self.smem_bytes = int(min(200 * 1024, max((p.fold.R + 7) // 8 * 8 * p.fold.NN * 64 for p in self.preps)))
         descs = np.zeros(len(self.preps), DESC_DTYPE)
         for i, p in enumerate(self.preps):
-            p.coeffs = torch.empty((4, p.N, 2 * p.K), dtype=torch.float64, device=dev)
+            p.slopes = torch.empty((p.N, 2 * p.K), dtype=torch.float64, device=dev)
             p.W = torch.empty((max(p.seg.nseg, 1), p.fold.R, p.fold.NN, 4), dtype=torch.complex128, device=dev)
             p.Bpk = None
             if self.precision == "mixed":
@@ -201,10 +201,7 @@ class BatchedInterpolatedModeSum:
         for i, p in enumerate(self.preps):
             st = side[i % len(side)].cuda_stream
             p.st = st
-            _lib.call("few_spline_build_factored", _ptr(p.fac), _ptr(p.teuk), 2 * p.K, 2, p.K, 1, 2 * p.K, p.N,
-                      _ptr(p.coeffs), _lib.FEW_LAYOUT_KNOT_MAJOR, st)
-            _lib.call("few_fold_coeffs", _ptr(p.coeffs), _ptr(p.ylm), _ptr(p.fold.d_key_ptr), _ptr(p.fold.d_key_list),
-                      p.K, p.N, p.seg.nseg, p.fold.R, p.fold.NN, _ptr(p.W), st)
+            fold_amplitudes(p, p.slopes, p.W, st)
             if p.Bpk is not None:
                 _lib.call("few_fold_mixed", _ptr(p.W), _ptr(p.t_dev), p.seg.nseg, p.fold.R, p.fold.NN, _ptr(p.Bpk),
                           st)

@@ -44,6 +44,7 @@ cudaError_t ensure_smem_attr(const void *kernel, int bytes);
 int fold_plan(const int *m, const int *k, const int *n, int K, int max_rows, int max_keys, int *row_m,
               int *row_k, int *dims, int *key_ptr, int *key_list);
 int spline_factor(const double *x, int N, double *fac);
+int spline_overlap(const double *fac, int N);
 int segment_plan(const double *h_t, const double *phase_t, int init_len, int out_len, double dt,
                  int chunk, int max_units, int *seg_start, double *seg_info, int *units, int *counts);
 

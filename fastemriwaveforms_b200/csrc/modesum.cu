@@ -81,6 +81,82 @@ __global__ void __launch_bounds__(256) k_fold_coeffs(const double *__restrict__ 
     for (int c = 0; c < 4; ++c) w[c] = acc[c];
 }
 
+// The same from the knot values and slopes of the amplitudes, (N, K) complex each: a
+// contributor's four coefficients are formed on the way, in the operations of the
+// spline build, so W has the same bits while a quarter of the bytes is read (the
+// coefficients are neither written nor read).  A thread takes one key through kFoldRun
+// segments, whose inner knots it reads once.  Bound by the latency of the rows' loads:
+// one year, 3843 modes: 61 us (112 us from the coefficients; 65 us a segment at a
+// time, 63 us by four).
+constexpr int kFoldRun = 2;
+
+__global__ void __launch_bounds__(128, 5) k_fold_slopes(const double2 *__restrict__ y, const double2 *__restrict__ sl,
+                                                        const double *__restrict__ fac,
+                                                        const double2 *__restrict__ ylms,
+                                                        const int *__restrict__ key_ptr,
+                                                        const int *__restrict__ key_list, int K, int nseg, int nkeys,
+                                                        double2 *__restrict__ W)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= nkeys) return;
+    const int s0 = blockIdx.y * kFoldRun, n = min(kFoldRun, nseg - s0);
+    double2 acc[kFoldRun][4];
+    double ih[kFoldRun];
+#pragma unroll
+    for (int i = 0; i < kFoldRun; ++i) {
+        ih[i] = __ldg(fac + (long long)kFacWidth * (s0 + min(i, n - 1)) + 6);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[i][c] = make_double2(0.0, 0.0);
+    }
+    const int b = key_ptr[q], e = key_ptr[q + 1];
+    int next = b < e ? key_list[b] : 0;
+    for (int it = b; it < e; ++it) {
+        const int code = next, j = code >> 1;
+        if (it + 1 < e) next = key_list[it + 1];
+        const bool minus = code & 1;
+        const double2 Y = minus ? ylms[K + j] : ylms[j];
+        const double2 *yj = y + (long long)s0 * K + j, *sj = sl + (long long)s0 * K + j;
+        double2 v[kFoldRun + 1], d[kFoldRun + 1];
+#pragma unroll
+        for (int i = 0; i <= kFoldRun; ++i) {
+            v[i] = yj[(long long)min(i, n) * K];
+            d[i] = sj[(long long)min(i, n) * K];
+        }
+#pragma unroll
+        for (int i = 0; i < kFoldRun; ++i) {
+            double2 co[4];
+            co[0] = v[i];
+            co[1] = d[i];
+            {
+                const double dl = (v[i + 1].x - v[i].x) * ih[i];
+                const double tt = (d[i].x + d[i + 1].x - 2 * dl) * ih[i];
+                co[2].x = (dl - d[i].x) * ih[i] - tt;
+                co[3].x = tt * ih[i];
+            }
+            {
+                const double dl = (v[i + 1].y - v[i].y) * ih[i];
+                const double tt = (d[i].y + d[i + 1].y - 2 * dl) * ih[i];
+                co[2].y = (dl - d[i].y) * ih[i] - tt;
+                co[3].y = tt * ih[i];
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const double ar = co[c].x, ai = minus ? -co[c].y : co[c].y;
+                acc[i][c].x = fma(Y.x, ar, fma(-Y.y, ai, acc[i][c].x));
+                acc[i][c].y = fma(Y.x, ai, fma(Y.y, ar, acc[i][c].y));
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kFoldRun; ++i) {
+        if (i < n) {
+            double2 *w = W + ((long long)(s0 + i) * nkeys + q) * 4;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) w[c] = acc[i][c];
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Sum.
 // ---------------------------------------------------------------------------
@@ -493,6 +569,26 @@ extern "C" int few_fold_coeffs(const double *coeffs, const void *ylms, const int
         return few::fail(FEW_ERR_SIZE, "few_fold_coeffs: bad sizes");
     return few::launch_fold(coeffs, (const double2 *)ylms, key_ptr, key_list, K, N, nseg, R, NN, (double2 *)W,
                             (cudaStream_t)stream);
+}
+
+extern "C" int few_fold_slopes(const void *y, const void *slopes, const double *fac, const void *ylms,
+                               const int *key_ptr, const int *key_list, int K, int N, int nseg, int R, int NN, void *W,
+                               void *stream)
+{
+    few::clear_error();
+    if (!y || !slopes || !fac || !ylms || !key_ptr || !key_list || !W)
+        return few::fail(FEW_ERR_ARG, "few_fold_slopes: null pointer");
+    if (K < 1 || N < 2 || nseg < 0 || nseg > N - 1 || R < 1 || NN < 1)
+        return few::fail(FEW_ERR_SIZE, "few_fold_slopes: bad sizes");
+    if (nseg == 0) return FEW_OK;
+    const int nkeys = R * NN;
+    dim3 grid((nkeys + 127) / 128, (nseg + few::kFoldRun - 1) / few::kFoldRun);
+    if (grid.y > 65535) return few::fail(FEW_ERR_SIZE, "few_fold_slopes: %d segments are too many", nseg);
+    few::k_fold_slopes<<<grid, 128, 0, (cudaStream_t)stream>>>(
+        (const double2 *)y, (const double2 *)slopes, fac, (const double2 *)ylms, key_ptr, key_list, K, nseg, nkeys,
+        (double2 *)W);
+    FEW_LAUNCH_CHECK("k_fold_slopes");
+    return FEW_OK;
 }
 
 extern "C" int few_sum_batched(const few_wave_desc *descs, int nwave, const int *units4, int nunits, int smem_bytes,

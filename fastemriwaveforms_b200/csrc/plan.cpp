@@ -220,7 +220,49 @@ int spline_factor(const double *x, int N, double *fac)
     return FEW_OK;
 }
 
+// Rows after which the sweeps of the factorization have forgotten their start: the
+// smallest w such that every product of w successive factors, forward (-lo_i/den_i)
+// and backward (-c'_i), is below 2^-60.  Large when some knots are very uneven.
+int spline_overlap(const double *fac, int N)
+{
+    if (!fac) return fail(FEW_ERR_ARG, "few_spline_overlap: null pointer");
+    if (N < 4) return fail(FEW_ERR_SIZE, "few_spline_overlap: length=%d < 4", N);
+    const int W = kFacWidth;
+    const double tol = 0x1p-60;
+    int w = 1;
+    for (int way = 0; way < 2; ++way) {
+        // runs [a, i) of factors whose product is just below tol, by two ends; a zero
+        // factor (the first row, or the last) ends every run across it
+        int a = 1;
+        double p = 1.0;
+        for (int i = 1; i <= N - 2; ++i) {
+            const double f = std::fabs(way == 0 ? fac[W * i] * fac[W * i + 1] : fac[W * i + 2]);
+            if (f == 0.0) {
+                w = std::max(w, i - a);
+                a = i + 1;
+                p = 1.0;
+                continue;
+            }
+            p *= f;
+            while (a < i) {  // the first factor may go while the rest stays below tol
+                const double g = std::fabs(way == 0 ? fac[W * a] * fac[W * a + 1] : fac[W * a + 2]);
+                if (!(p / g < tol)) break;
+                p /= g;
+                ++a;
+            }
+            w = std::max(w, i - a + 1);
+        }
+    }
+    return w;
+}
+
 }  // namespace few
+
+extern "C" int few_spline_overlap(const double *fac, int N)
+{
+    few::clear_error();
+    return few::spline_overlap(fac, N);
+}
 
 extern "C" int few_spline_factor(const double *t, int N, double *fac)
 {

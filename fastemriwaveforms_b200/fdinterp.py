@@ -28,7 +28,7 @@ import torch
 
 from . import _lib
 from .geodesic import MTSUN_SI, fundamental_frequencies_into
-from .summation import SummationBase, _device, _input, _ptr, _stream, _to_device, _to_host, spline_factor_table
+from .summation import SummationBase, _device, _input, _ptr, _stream, _to_device, _to_host, build_splines, spline_factor
 
 DENSE_POINTS = 5000  # dense grid of the turnover search (fdinterp.py:266)
 
@@ -115,10 +115,9 @@ class FDInterpolatedModeSum(SummationBase):
 
         # 2. splines: amplitudes (4, N, 2K) knot-major, frequencies (4, N, 3)
         amp = torch.empty((4, N, 2 * K), dtype=torch.float64, device=dev)
-        fac = spline_factor_table(t_h, dev)
+        fac, overlap = spline_factor(t_h, dev)
         tv = torch.view_as_real(teuk)
-        _lib.call("few_spline_build_factored", _ptr(fac), _ptr(tv), 2 * K, 2, K, 1, 2 * K, N, _ptr(amp),
-                  _lib.FEW_LAYOUT_KNOT_MAJOR, st)
+        build_splines(fac, overlap, _ptr(tv), (2 * K, 2, K, 1), 2 * K, N, amp, st)
         fco = torch.empty((4, N, 3), dtype=torch.float64, device=dev)
         _lib.call("few_spline_build", _ptr(t_d), 0, _ptr(fk), 1, N, 3, 0, 3, N, _ptr(fco), _lib.FEW_LAYOUT_KNOT_MAJOR,
                   st)

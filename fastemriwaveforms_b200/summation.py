@@ -149,13 +149,53 @@ def _ptr(t: torch.Tensor) -> int:
     return t.data_ptr()
 
 
-def spline_factor_table(h_t: np.ndarray, device) -> torch.Tensor:
-    """Device copy of the not-a-knot factorization for knots h_t (few_spline_factor)."""
+# From this many knots on, the one-pass spline builds are the faster ones (below, the
+# chunks of k_spline_build_factored are shorter than a run and its overlaps: 8.1
+# against 10.8 us at 100 knots of 400 series, 13.4 against 11.4 us at 200).
+ONE_PASS_KNOTS = 150
+
+
+def spline_factor(h_t: np.ndarray, device):
+    """Device copy of the not-a-knot factorization for knots h_t (few_spline_factor),
+    and its overlap (few_spline_overlap; 0 where the one-pass builds are not used)."""
     h_t = np.ascontiguousarray(h_t, dtype=np.float64)
     N = len(h_t)
     fac = np.zeros(_lib.FEW_FAC_WIDTH * (N + 1), np.float64)
     _lib.call("few_spline_factor", h_t.ctypes.data, N, fac.ctypes.data)
-    return torch.from_numpy(fac).pin_memory().to(device, non_blocking=True)
+    overlap = 0
+    if N >= ONE_PASS_KNOTS:
+        lib = _lib.load()
+        overlap = int(lib.few_spline_overlap(fac.ctypes.data, N))
+        if not 1 <= overlap <= lib.few_spline_max_overlap():
+            overlap = 0
+    return torch.from_numpy(fac).pin_memory().to(device, non_blocking=True), overlap
+
+
+def spline_factor_table(h_t: np.ndarray, device) -> torch.Tensor:
+    """The factorization alone."""
+    return spline_factor(h_t, device)[0]
+
+
+def build_splines(fac, overlap, y_ptr, y_strides, ninterps, length, coeffs, st):
+    """Spline coefficients (4, length, ninterps) on shared knots; y_strides =
+    (knot stride, series stride, split, split offset) of few_spline_build."""
+    if overlap:
+        _lib.call("few_spline_build_chunked", _ptr(fac), overlap, y_ptr, *y_strides, ninterps, length, _ptr(coeffs),
+                  _lib.FEW_LAYOUT_KNOT_MAJOR, st)
+    else:
+        _lib.call("few_spline_build_factored", _ptr(fac), y_ptr, *y_strides, ninterps, length, _ptr(coeffs),
+                  _lib.FEW_LAYOUT_KNOT_MAJOR, st)
+
+
+def fold_amplitudes(p, slopes, W, st, between=None):
+    """Folded coefficients W of a prepared call on stream st, through the slopes
+    (N, 2K) of its amplitude splines; between: a CUDA event recorded after these."""
+    fold, seg, N, K = p.fold, p.seg, p.N, p.K
+    _lib.call("few_spline_slopes", _ptr(p.fac), _ptr(p.teuk), 2 * K, N, _ptr(slopes), st)
+    if between:
+        between.record()
+    _lib.call("few_fold_slopes", _ptr(p.teuk), _ptr(slopes), _ptr(p.fac), _ptr(p.ylm), _ptr(fold.d_key_ptr),
+              _ptr(fold.d_key_list), K, N, seg.nseg, fold.R, fold.NN, _ptr(W), st)
 
 
 class CubicSplineInterpolant:
@@ -199,16 +239,19 @@ class CubicSplineInterpolant:
             raise ValueError("t and y_all must have the same length along the time axis.")
         if self.length < 4:
             raise ValueError("not-a-knot cubic splines need at least 4 knots.")
-        if not bool((t_dev[..., 1:] > t_dev[..., :-1]).all()):
+        # shared knots are factored on the host, so their order is checked there too
+        t_h = _to_host(t_arr, np.float64) if t_rs == 0 else None
+        increases = (t_h[1:] > t_h[:-1]).all() if t_rs == 0 else (t_dev[..., 1:] > t_dev[..., :-1]).all()
+        if not bool(increases):
             raise ValueError("t must increase strictly along the time axis.")
         self._t_knots = t_dev
         self._t_rs = t_rs
         coeffs = torch.empty((4, self.length, self.ninterps), dtype=torch.float64, device=dev)
         if t_rs == 0:
             # shared knots: factor once on the host, sweep per series on the device
-            fac = spline_factor_table(t_dev.cpu().numpy(), dev)
-            _lib.call("few_spline_build_factored", _ptr(fac), _ptr(y), 1, self.length, self.ninterps, 0,
-                      self.ninterps, self.length, _ptr(coeffs), _lib.FEW_LAYOUT_KNOT_MAJOR, _stream(dev))
+            fac, overlap = spline_factor(t_h, dev)
+            build_splines(fac, overlap, _ptr(y), (1, self.length, self.ninterps, 0), self.ninterps, self.length, coeffs,
+                          _stream(dev))
         else:
             _lib.call("few_spline_build", _ptr(t_dev), t_rs, _ptr(y), 1, self.length, self.ninterps, 0,
                       self.ninterps, self.length, _ptr(coeffs), _lib.FEW_LAYOUT_KNOT_MAJOR, _stream(dev))
@@ -587,19 +630,12 @@ class InterpolatedModeSum(SummationBase):
         output samples) and each finished slice is copied to `host_out` on a
         download stream while the next part computes."""
         fold, seg, N, K, st = p.fold, p.seg, p.N, p.K, p.st
-        coeffs = torch.empty((4, N, 2 * K), dtype=torch.float64, device=p.dev)
+        slopes = torch.empty((N, 2 * K), dtype=torch.float64, device=p.dev)
         W = torch.empty((max(seg.nseg, 1), fold.R, fold.NN, 4), dtype=torch.complex128, device=p.dev)
         ev = [torch.cuda.Event(enable_timing=True) for _ in range(4)] if self.record_stages else None
         if ev:
             ev[0].record()
-        # amplitude splines straight from the (N, K) complex array: real parts are
-        # interpolants 0..K-1, imaginary parts K..2K-1 (interpolatedmodesum.py:331-337)
-        _lib.call("few_spline_build_factored", _ptr(p.fac), _ptr(p.teuk), 2 * K, 2, K, 1, 2 * K, N, _ptr(coeffs),
-                  _lib.FEW_LAYOUT_KNOT_MAJOR, st)
-        if ev:
-            ev[1].record()
-        _lib.call("few_fold_coeffs", _ptr(coeffs), _ptr(p.ylm), _ptr(fold.d_key_ptr), _ptr(fold.d_key_list), K, N,
-                  seg.nseg, fold.R, fold.NN, _ptr(W), st)
+        fold_amplitudes(p, slopes, W, st, ev[1] if ev else None)
         if ev:
             ev[2].record()
         if self.precision == "mixed":
@@ -757,7 +793,7 @@ class InterpolatedModeSum(SummationBase):
 
     def stage_times(self) -> dict:
         """Kernel times (ms) of the last call with ``record_stages`` set:
-        spline build, fold and sum (three back-to-back launches)."""
+        amplitude splines, fold and sum (back-to-back launches)."""
         ev = self._stage_events
         if ev is None:
             return {}

@@ -166,6 +166,25 @@ FEW_API int few_spline_build_factored(const double *fac, const double *y, long l
                                       long long y_interp_stride, int y_split, long long y_split_offset,
                                       int ninterps, int length, double *coeffs, int layout, void *stream);
 
+/* Rows after which the sweeps of a factorization fac [host] (few_spline_factor, N
+ * knots) have forgotten their start: every product of that many of their factors is
+ * below 2^-60 (30 to 40 on ordinary knots).  Negative: an error status. */
+FEW_API int few_spline_overlap(const double *fac, int N);
+
+/* Largest overlap few_spline_build_chunked takes. */
+FEW_API int few_spline_max_overlap(void);
+
+/* few_spline_build_factored in one pass over independent runs of knots, for
+ * 1 <= overlap <= few_spline_max_overlap() (few_spline_overlap's, or more). */
+FEW_API int few_spline_build_chunked(const double *fac, int overlap, const double *y, long long y_knot_stride,
+                                     long long y_interp_stride, int y_split, long long y_split_offset, int ninterps,
+                                     int length, double *coeffs, int layout, void *stream);
+
+/* The slopes at the knots of few_spline_build_factored's splines alone (the c1 plane,
+ * same bits): y, slopes [device] (length, ninterps), not overlapping. */
+FEW_API int few_spline_slopes(const double *fac, const double *y, int ninterps, int length, double *slopes,
+                              void *stream);
+
 /* Spline evaluation (CubicSplineInterpolant.__call__, interpolatedmodesum.py:161-257).
  * t [device]: knots, interpolant p uses t + p*t_row_stride (0 = shared).
  * coeffs [device] (4, length, ninterps).  tnew [device]: point j of
@@ -220,6 +239,13 @@ FEW_API int few_segment_plan(const double *h_t, const double *phase_t, int init_
  * W [device] (nseg, R, NN, 4) complex. */
 FEW_API int few_fold_coeffs(const double *coeffs, const void *ylms, const int *key_ptr, const int *key_list,
                     int K, int N, int nseg, int R, int NN, void *W, void *stream);
+
+/* few_fold_coeffs (same bits) from the amplitudes y and their slopes [device] (N, K)
+ * complex (few_spline_slopes with ninterps = 2K) instead of few_spline_build_factored's
+ * coefficients; fac [device]. */
+FEW_API int few_fold_slopes(const void *y, const void *slopes, const double *fac, const void *ylms,
+                            const int *key_ptr, const int *key_list, int K, int N, int nseg, int R, int NN, void *W,
+                            void *stream);
 
 /* Accumulates the folded sum into wf [device] (out_len,) complex:
  * wf[i] += sum_{r,c'} (sum_c x^c W[s][r][c'][c]) exp(-i phase_{r,c'}(t_i)),
