@@ -41,7 +41,6 @@ namespace few {
 namespace {
 
 constexpr int kSumThreads = 256;
-constexpr int kRowBlock = 8;                   // rows held in registers at once
 constexpr int kSmemBudget = 200 * 1024;        // dynamic shared memory for W per CTA
 
 // ---------------------------------------------------------------------------
@@ -169,18 +168,134 @@ struct SumArgs {
     const int *row_m;
     const int *row_k;
     int N, R, nlo, NN;
-    int rows_per_pass;
+    int blocks_per_pass;  // row blocks whose coefficients are in shared memory at once
     int use_theta;
     double dt;
 };
 
-// Rows per pass of the folded sum: all R when their blocks of RB rows fit in
-// smem_bytes, else the most whole blocks that fit (0 if not even one does).
-__host__ __device__ inline int sum_rows_per_pass(int R, int NN, int RB, int smem_bytes)
+// The rows go through the registers in ceil(R / RB) blocks of nearly equal size (RB
+// rows at most); block b starts at row row_block(b).
+__host__ __device__ inline int row_blocks(int R, int RB) { return (R + RB - 1) / RB; }
+__host__ __device__ inline int row_block(int b, int R, int nblk) { return (int)((long long)b * R / nblk); }
+
+// Blocks per pass: all when their coefficients fit in smem_bytes, else the most that
+// surely fit (0 if not even one does).
+__host__ __device__ inline int sum_blocks_per_pass(int R, int NN, int RB, int smem_bytes)
 {
-    const int fit = smem_bytes / (NN * 4 * (int)sizeof(double2));  // rows whose coefficients fit
-    if ((R + RB - 1) / RB * RB <= fit) return R;
-    return fit / RB * RB;
+    const int nblk = row_blocks(R, RB), fit = smem_bytes / (NN * 4 * (int)sizeof(double2));  // rows that fit
+    return R <= fit ? nblk : fit / ((R + nblk - 1) / nblk);
+}
+
+// A thread's samples between row blocks.
+template <int SPT>
+struct SumSamples {
+    double x[SPT], Pp[SPT], Pr[SPT], Pt[SPT];
+    double2 Ep[SPT], Er[SPT], Et[SPT], V0[SPT], h[SPT];
+};
+
+// One block of NR rows over all columns.  NR is a compile-time count, so the column
+// loop has no test per row: with one the rows' loads and chains cannot be
+// interleaved, and each row waits for its own shared-memory reads (one year, 3843
+// modes: exact 5.73 ms with the test, 4.22 without; faithful 7.13 and 6.65; 363 modes
+// of 63 rows: 1.09 and 0.88).
+template <int NR, bool FAITHFUL, int SPT, bool THETA>
+__device__ __forceinline__ void sum_rows(const double2 *__restrict__ wblk, const int *rm, const int *rk, int nlo, int NN,
+                                         bool theta, const volatile double *park_ep, const volatile double *park_pp,
+                                         SumSamples<SPT> &m)
+{
+    double2 U[SPT][NR];
+    double S12[SPT][NR];
+    double2 Epb[SPT];
+    double Ppb[SPT];
+#pragma unroll
+    for (int sm = 0; sm < SPT; ++sm) {
+        const int slot = sm * kSumThreads + threadIdx.x;
+        Epb[sm] = FAITHFUL ? make_double2(park_ep[2 * slot], park_ep[2 * slot + 1]) : m.Ep[sm];
+        Ppb[sm] = FAITHFUL ? park_pp[slot] : m.Pp[sm];
+    }
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+        const int mm = rm[q], kk = rk[q];
+#pragma unroll
+        for (int sm = 0; sm < SPT; ++sm) {
+            double2 uu = cpow_int(Epb[sm], mm);
+            if (theta && kk) uu = cmul(uu, cpow_int(m.Et[sm], kk));
+            S12[sm][q] = 0.0;
+            if (FAITHFUL) {
+                const double dm = (double)mm;
+                const double p1 = rmul(dm, Ppb[sm]);
+                const double e1 = fma(dm, Ppb[sm], -p1);
+                if (THETA) {
+                    const double dk = (double)kk;
+                    const double p2 = rmul(dk, m.Pt[sm]);
+                    const double e2 = fma(dk, m.Pt[sm], -p2);
+                    const double s12 = radd(p1, p2);
+                    const double e12 = two_sum_err(p1, p2, s12);
+                    uu = crot_small(uu, (e1 + e2) + e12);
+                    S12[sm][q] = s12;
+                } else {
+                    // fl(p1 + 0) = p1 and its TwoSum error is 0
+                    uu = crot_small(uu, e1);
+                    S12[sm][q] = p1;
+                }
+            }
+            U[sm][q] = uu;
+        }
+    }
+    double2 v[SPT];
+#pragma unroll
+    for (int sm = 0; sm < SPT; ++sm) v[sm] = FAITHFUL ? cpow_int(m.Er[sm], nlo) : m.V0[sm];
+    for (int c = 0; c < NN; ++c) {
+        double2 vv[SPT], T[SPT];
+        double p3[SPT];
+#pragma unroll
+        for (int sm = 0; sm < SPT; ++sm) {
+            vv[sm] = v[sm];
+            p3[sm] = 0.0;
+            if (FAITHFUL) {
+                const double dn = (double)(nlo + c);
+                p3[sm] = rmul(dn, m.Pr[sm]);
+                vv[sm] = crot_small(v[sm], fma(dn, m.Pr[sm], -p3[sm]));
+            }
+            T[sm] = make_double2(0.0, 0.0);
+        }
+        const double2 *w = wblk + c * (NR * 4);
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+            const double2 w0 = w[4 * q], w1 = w[4 * q + 1], w2 = w[4 * q + 2], w3 = w[4 * q + 3];
+#pragma unroll
+            for (int sm = 0; sm < SPT; ++sm) {
+                double2 Wx;
+                Wx.x = fma(fma(fma(w3.x, m.x[sm], w2.x), m.x[sm], w1.x), m.x[sm], w0.x);
+                Wx.y = fma(fma(fma(w3.y, m.x[sm], w2.y), m.x[sm], w1.y), m.x[sm], w0.y);
+                if (FAITHFUL) {
+                    const double sp = radd(S12[sm][q], p3[sm]);
+                    Wx = crot_small(Wx, two_sum_err(S12[sm][q], p3[sm], sp));
+                }
+                T[sm].x = fma(U[sm][q].x, Wx.x, fma(-U[sm][q].y, Wx.y, T[sm].x));
+                T[sm].y = fma(U[sm][q].x, Wx.y, fma(U[sm][q].y, Wx.x, T[sm].y));
+            }
+        }
+#pragma unroll
+        for (int sm = 0; sm < SPT; ++sm) {
+            m.h[sm].x = fma(vv[sm].x, T[sm].x, fma(-vv[sm].y, T[sm].y, m.h[sm].x));
+            m.h[sm].y = fma(vv[sm].x, T[sm].y, fma(vv[sm].y, T[sm].x, m.h[sm].y));
+            v[sm] = cmul(v[sm], m.Er[sm]);
+        }
+    }
+}
+
+// sum_rows with the block's row count (1..NR) made a compile-time one.
+template <int NR, bool FAITHFUL, int SPT, bool THETA>
+__device__ __forceinline__ void sum_rows_of(int rows, const double2 *wblk, const int *rm, const int *rk, int nlo, int NN,
+                                            bool theta, const volatile double *park_ep, const volatile double *park_pp,
+                                            SumSamples<SPT> &m)
+{
+    if (rows == NR) {
+        sum_rows<NR, FAITHFUL, SPT, THETA>(wblk, rm, rk, nlo, NN, theta, park_ep, park_pp, m);
+    } else if constexpr (NR > 1) {
+        sum_rows_of<NR - 1, FAITHFUL, SPT, THETA>(rows, wblk, rm, rk, nlo, NN, theta, park_ep, park_pp, m);
+    }
 }
 
 // One work unit (samples [lo, hi) of segment seg) of the folded sum; the
@@ -196,7 +311,7 @@ __device__ __forceinline__ void sum_unit(const SumArgs &a, int seg, int lo, int 
                                          double *s_pc)
 {
     const double t0 = a.seg_info[3 * seg], pt0 = a.seg_info[3 * seg + 1], pw = a.seg_info[3 * seg + 2];
-    const int R = a.R, NN = a.NN, nlo = a.nlo;
+    const int R = a.R, NN = a.NN, nlo = a.nlo, nblk = row_blocks(R, RB);
     const long long nps = (long long)(a.N - 1) * 3;
     const bool theta = THETA && a.use_theta;
     // The faithful form parks Phi_phi and e^{-i Phi_phi}, needed only at each
@@ -219,154 +334,65 @@ __device__ __forceinline__ void sum_unit(const SumArgs &a, int seg, int lo, int 
         s_pc[threadIdx.x] = a.pc[c * nps + (long long)seg * 3 + q];
     }
 
-    for (int r0 = 0; r0 < R; r0 += a.rows_per_pass) {
-        const int nrp = min(a.rows_per_pass, R - r0);
+    for (int b0 = 0; b0 < nblk; b0 += a.blocks_per_pass) {
+        const int b1 = min(b0 + a.blocks_per_pass, nblk), r0 = row_block(b0, R, nblk);
         __syncthreads();  // previous pass finished reading sW
-        {
-            // rows (row, n', c) in global order -> blocks of RB rows, each laid out
-            // (n', row in block, c): the 4 RB coefficients one column needs are
-            // contiguous (the last block of a pass may be partly unused)
-            const double2 *src = a.W + ((long long)seg * R + r0) * NN * 4;
-            const int count = nrp * NN * 4;
+        // rows (row, n', c) in global order -> blocks of rows, each laid out (n', row
+        // in block, c): the coefficients one column needs are contiguous
+        for (int b = b0; b < b1; ++b) {
+            const int ra = row_block(b, R, nblk), nr = row_block(b + 1, R, nblk) - ra;
+            const double2 *src = a.W + ((long long)seg * R + ra) * NN * 4;
+            double2 *dst = sW + (ra - r0) * NN * 4;
+            const int count = nr * NN * 4;
             for (int e = threadIdx.x; e < count; e += blockDim.x) {
-                const int rr = e / (NN * 4), rem = e - rr * (NN * 4);
-                const int blk = rr / RB, q = rr - blk * RB;
-                sW[((blk * NN) + (rem >> 2)) * (RB * 4) + q * 4 + (rem & 3)] = src[e];
+                const int q = e / (NN * 4), rem = e - q * (NN * 4);
+                dst[((rem >> 2) * nr + q) * 4 + (rem & 3)] = src[e];
             }
         }
         __syncthreads();
         for (int ib = lo + threadIdx.x; ib < hi; ib += SPT * blockDim.x) {
-            double x[SPT], Pp[SPT], Pr[SPT], Pt[SPT];
-            double2 Ep[SPT], Er[SPT], Et[SPT], V0[SPT], h[SPT];
+            SumSamples<SPT> m;
 #pragma unroll
             for (int sm = 0; sm < SPT; ++sm) {
                 // a sample past the end repeats the first one; its result is dropped
                 const int i = (ib + sm * (int)blockDim.x < hi) ? ib + sm * (int)blockDim.x : ib;
                 // Sample time and phases exactly as interpolate.cu:626-644.
                 const double t = rmul(a.dt, (double)i);
-                x[sm] = rsub(t, t0);
+                m.x[sm] = rsub(t, t0);
                 const double s = __ddiv_rn(rsub(t, pt0), pw);
                 const double s1 = rsub(1.0, s);
-                Pp[sm] = phase_poly(s_pc, s, s1);
-                Pr[sm] = phase_poly(s_pc + 16, s, s1);
-                Pt[sm] = theta ? phase_poly(s_pc + 8, s, s1) : 0.0;
+                m.Pp[sm] = phase_poly(s_pc, s, s1);
+                m.Pr[sm] = phase_poly(s_pc + 16, s, s1);
+                m.Pt[sm] = theta ? phase_poly(s_pc + 8, s, s1) : 0.0;
                 double sn, cs;
-                sincos(Pp[sm], &sn, &cs);
-                Ep[sm] = make_double2(cs, -sn);
+                sincos(m.Pp[sm], &sn, &cs);
+                m.Ep[sm] = make_double2(cs, -sn);
                 if (FAITHFUL) {
-                    s_park_ep[sm * kSumThreads + threadIdx.x] = Ep[sm];
-                    s_park_pp[sm * kSumThreads + threadIdx.x] = Pp[sm];
+                    s_park_ep[sm * kSumThreads + threadIdx.x] = m.Ep[sm];
+                    s_park_pp[sm * kSumThreads + threadIdx.x] = m.Pp[sm];
                 }
-                sincos(Pr[sm], &sn, &cs);
-                Er[sm] = make_double2(cs, -sn);
-                Et[sm] = make_double2(1.0, 0.0);
+                sincos(m.Pr[sm], &sn, &cs);
+                m.Er[sm] = make_double2(cs, -sn);
+                m.Et[sm] = make_double2(1.0, 0.0);
                 if (theta) {
-                    sincos(Pt[sm], &sn, &cs);
-                    Et[sm] = make_double2(cs, -sn);
+                    sincos(m.Pt[sm], &sn, &cs);
+                    m.Et[sm] = make_double2(cs, -sn);
                 }
-                if (!FAITHFUL) V0[sm] = cpow_int(Er[sm], nlo);
-                h[sm] = make_double2(0.0, 0.0);
+                if (!FAITHFUL) m.V0[sm] = cpow_int(m.Er[sm], nlo);
+                m.h[sm] = make_double2(0.0, 0.0);
             }
-
-            for (int rb = 0; rb < nrp; rb += RB) {
-                double2 U[SPT][RB];
-                double S12[SPT][RB];
-                double2 Epb[SPT];
-                double Ppb[SPT];
-#pragma unroll
-                for (int sm = 0; sm < SPT; ++sm) {
-                    const int slot = sm * kSumThreads + threadIdx.x;
-                    Epb[sm] = FAITHFUL ? make_double2(park_ep[2 * slot], park_ep[2 * slot + 1]) : Ep[sm];
-                    Ppb[sm] = FAITHFUL ? park_pp[slot] : Pp[sm];
-                }
-#pragma unroll
-                for (int q = 0; q < RB; ++q) {
-#pragma unroll
-                    for (int sm = 0; sm < SPT; ++sm) {
-                        U[sm][q] = make_double2(0.0, 0.0);
-                        S12[sm][q] = 0.0;
-                    }
-                    if (rb + q < nrp) {
-                        const int mm = s_rm[r0 + rb + q], kk = s_rk[r0 + rb + q];
-#pragma unroll
-                        for (int sm = 0; sm < SPT; ++sm) {
-                            double2 uu = cpow_int(Epb[sm], mm);
-                            if (theta && kk) uu = cmul(uu, cpow_int(Et[sm], kk));
-                            if (FAITHFUL) {
-                                const double dm = (double)mm;
-                                const double p1 = rmul(dm, Ppb[sm]);
-                                const double e1 = fma(dm, Ppb[sm], -p1);
-                                if (THETA) {
-                                    const double dk = (double)kk;
-                                    const double p2 = rmul(dk, Pt[sm]);
-                                    const double e2 = fma(dk, Pt[sm], -p2);
-                                    const double s12 = radd(p1, p2);
-                                    const double e12 = two_sum_err(p1, p2, s12);
-                                    uu = crot_small(uu, (e1 + e2) + e12);
-                                    S12[sm][q] = s12;
-                                } else {
-                                    // fl(p1 + 0) = p1 and its TwoSum error is 0
-                                    uu = crot_small(uu, e1);
-                                    S12[sm][q] = p1;
-                                }
-                            }
-                            U[sm][q] = uu;
-                        }
-                    }
-                }
-                double2 v[SPT];
-#pragma unroll
-                for (int sm = 0; sm < SPT; ++sm) v[sm] = FAITHFUL ? cpow_int(Er[sm], nlo) : V0[sm];
-                const double2 *wrow = sW + (long long)rb * NN * 4;
-                for (int c = 0; c < NN; ++c) {
-                    double2 vv[SPT], T[SPT];
-                    double p3[SPT];
-#pragma unroll
-                    for (int sm = 0; sm < SPT; ++sm) {
-                        vv[sm] = v[sm];
-                        p3[sm] = 0.0;
-                        if (FAITHFUL) {
-                            const double dn = (double)(nlo + c);
-                            p3[sm] = rmul(dn, Pr[sm]);
-                            vv[sm] = crot_small(v[sm], fma(dn, Pr[sm], -p3[sm]));
-                        }
-                        T[sm] = make_double2(0.0, 0.0);
-                    }
-                    const double2 *wc = wrow + c * (RB * 4);
-#pragma unroll
-                    for (int q = 0; q < RB; ++q) {
-                        if (rb + q < nrp) {
-                            const double2 *w = wc + q * 4;
-                            const double2 w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3];
-#pragma unroll
-                            for (int sm = 0; sm < SPT; ++sm) {
-                                double2 Wx;
-                                Wx.x = fma(fma(fma(w3.x, x[sm], w2.x), x[sm], w1.x), x[sm], w0.x);
-                                Wx.y = fma(fma(fma(w3.y, x[sm], w2.y), x[sm], w1.y), x[sm], w0.y);
-                                if (FAITHFUL) {
-                                    const double sp = radd(S12[sm][q], p3[sm]);
-                                    Wx = crot_small(Wx, two_sum_err(S12[sm][q], p3[sm], sp));
-                                }
-                                T[sm].x = fma(U[sm][q].x, Wx.x, fma(-U[sm][q].y, Wx.y, T[sm].x));
-                                T[sm].y = fma(U[sm][q].x, Wx.y, fma(U[sm][q].y, Wx.x, T[sm].y));
-                            }
-                        }
-                    }
-#pragma unroll
-                    for (int sm = 0; sm < SPT; ++sm) {
-                        h[sm].x = fma(vv[sm].x, T[sm].x, fma(-vv[sm].y, T[sm].y, h[sm].x));
-                        h[sm].y = fma(vv[sm].x, T[sm].y, fma(vv[sm].y, T[sm].x, h[sm].y));
-                        v[sm] = cmul(v[sm], Er[sm]);
-                    }
-                }
+            for (int b = b0; b < b1; ++b) {
+                const int ra = row_block(b, R, nblk), nr = row_block(b + 1, R, nblk) - ra;
+                sum_rows_of<RB, FAITHFUL, SPT, THETA>(nr, sW + (ra - r0) * NN * 4, s_rm + ra, s_rk + ra, nlo, NN, theta,
+                                                      park_ep, park_pp, m);
             }
 #pragma unroll
             for (int sm = 0; sm < SPT; ++sm) {
                 const int i = ib + sm * (int)blockDim.x;
                 if (i < hi) {
                     double2 o = a.wf[i];
-                    o.x += h[sm].x;
-                    o.y += h[sm].y;
+                    o.x += m.h[sm].x;
+                    o.y += m.h[sm].y;
                     a.wf[i] = o;
                 }
             }
@@ -416,7 +442,7 @@ __global__ void __launch_bounds__(kSumThreads, (SPT == 1 || RB <= 4) ? 2 : 1) k_
         a.NN = d.NN;
         a.use_theta = d.use_theta;
         a.dt = d.dt;
-        a.rows_per_pass = sum_rows_per_pass(d.R, d.NN, RB, smem_bytes);
+        a.blocks_per_pass = sum_blocks_per_pass(d.R, d.NN, RB, smem_bytes);
         sum_unit<RB, FAITHFUL, SPT, true>(a, units4[4 * u + 1], units4[4 * u + 2], units4[4 * u + 3],
                                     reinterpret_cast<double2 *>(smem_raw), s_rm, s_rk, s_pc);
         if (done) {  // completion time of the waveform: the latest of its units
@@ -441,14 +467,18 @@ int launch_sum_t(const SumArgs &a, int nunits, size_t smem, cudaStream_t st)
     return FEW_OK;
 }
 
-// Shape of the FP64 sum: rows held in registers (RB) x samples per thread (SPT).
+// Shape of the FP64 sum: rows held in registers at most (RB) x samples per thread
+// (SPT).
 struct SumShape {
     int rb, spt;
 };
 
-// Measured on B200 at the one-year 3843-mode waveform: faithful 8 rows x 2
-// samples per thread (8.65 ms vs 9.17 ms for 8x1), exact 4 rows x 1 sample
-// (6.32 ms vs 7.15 ms).  FEW_B200_SUM_SHAPE="RBxSPT" overrides both.
+// Measured on B200, one year, 3843 modes (R = 21 rows, NN = 61 columns): faithful 7
+// rows x 2 samples 6.65 ms (6.81 with 6 rows, 7.16 with 5, 7.06 at 8 x 1 and 4 x 1,
+// 7.09 at 4 x 2); exact 6 x 1 4.22 ms (4.18 with 7, 4.33 with 4, 4.33 at 8 x 2), and
+// 0.88 ms on 363 modes with k' != 0 (R = 63, NN = 11; 0.89 with 7).  FP64 pipe 70 %
+// busy in the faithful form.  FEW_B200_SUM_SHAPE="RBxSPT" overrides both: 4 rows, or 8
+// for the most that there is.
 SumShape sum_shape(int mode)
 {
     static const SumShape forced = [] {
@@ -456,12 +486,13 @@ SumShape sum_shape(int mode)
         const char *v = getenv("FEW_B200_SUM_SHAPE");
         if (v) {
             int rb = 0, spt = 0;
-            if (sscanf(v, "%dx%d", &rb, &spt) == 2 && (rb == 4 || rb == 8) && (spt == 1 || spt == 2)) sh = {rb, spt};
+            if (sscanf(v, "%dx%d", &rb, &spt) == 2 && (rb == 4 || rb == 8) && (spt == 1 || spt == 2))
+                sh = {rb == 4 ? 4 : (spt == 1 ? 6 : 7), spt};
         }
         return sh;
     }();
     if (forced.rb) return forced;
-    return mode == FEW_SUM_FAITHFUL ? SumShape{8, 2} : SumShape{4, 1};
+    return mode == FEW_SUM_FAITHFUL ? SumShape{7, 2} : SumShape{6, 1};
 }
 
 template <int RB, bool F, int SPT>
@@ -496,14 +527,14 @@ int launch_sum_folded_batched(const few_wave_desc *descs, const int *units4, int
     if (sh.rb == 4 && sh.spt == 2)
         return F ? launch_batched_t<4, true, 2>(descs, units4, nunits, smem_bytes, ctas, done, st)
                  : launch_batched_t<4, false, 2>(descs, units4, nunits, smem_bytes, ctas, done, st);
-    if (sh.rb == 8 && sh.spt == 2)
-        return F ? launch_batched_t<8, true, 2>(descs, units4, nunits, smem_bytes, ctas, done, st)
-                 : launch_batched_t<8, false, 2>(descs, units4, nunits, smem_bytes, ctas, done, st);
+    if (sh.rb == 7)
+        return F ? launch_batched_t<7, true, 2>(descs, units4, nunits, smem_bytes, ctas, done, st)
+                 : launch_batched_t<7, false, 2>(descs, units4, nunits, smem_bytes, ctas, done, st);
     if (sh.rb == 4)
         return F ? launch_batched_t<4, true, 1>(descs, units4, nunits, smem_bytes, ctas, done, st)
                  : launch_batched_t<4, false, 1>(descs, units4, nunits, smem_bytes, ctas, done, st);
-    return F ? launch_batched_t<8, true, 1>(descs, units4, nunits, smem_bytes, ctas, done, st)
-             : launch_batched_t<8, false, 1>(descs, units4, nunits, smem_bytes, ctas, done, st);
+    return F ? launch_batched_t<6, true, 1>(descs, units4, nunits, smem_bytes, ctas, done, st)
+             : launch_batched_t<6, false, 1>(descs, units4, nunits, smem_bytes, ctas, done, st);
 }
 
 int launch_fold(const double *coeffs, const double2 *ylms, const int *key_ptr, const int *key_list, int K, int N,
@@ -540,22 +571,22 @@ int launch_sum_folded(double2 *wf, const double2 *W, const double *pc, int N, co
     a.dt = dt;
     const long long row_bytes = (long long)NN * 4 * sizeof(double2);
     const SumShape sh = sum_shape(mode);
-    const int rpp = sum_rows_per_pass(R, NN, sh.rb, kSmemBudget);
-    if (rpp < 1)
+    const int nblk = row_blocks(R, sh.rb), bpp = sum_blocks_per_pass(R, NN, sh.rb, kSmemBudget);
+    if (bpp < 1)
         return fail(FEW_ERR_SIZE, "few_sum_folded: NN=%d too large for one row block in shared memory", NN);
-    a.rows_per_pass = rpp;
-    const size_t smem = (size_t)((rpp + sh.rb - 1) / sh.rb * sh.rb) * row_bytes;
+    a.blocks_per_pass = bpp;
+    const size_t smem = (size_t)std::min(R, bpp * ((R + nblk - 1) / nblk)) * row_bytes;
     if (sh.rb == 4 && sh.spt == 2)
         return mode == FEW_SUM_FAITHFUL ? launch_sum_t<4, true, 2>(a, nunits, smem, st)
                                         : launch_sum_t<4, false, 2>(a, nunits, smem, st);
-    if (sh.rb == 8 && sh.spt == 2)
-        return mode == FEW_SUM_FAITHFUL ? launch_sum_t<8, true, 2>(a, nunits, smem, st)
-                                        : launch_sum_t<8, false, 2>(a, nunits, smem, st);
+    if (sh.rb == 7)
+        return mode == FEW_SUM_FAITHFUL ? launch_sum_t<7, true, 2>(a, nunits, smem, st)
+                                        : launch_sum_t<7, false, 2>(a, nunits, smem, st);
     if (sh.rb == 4)
         return mode == FEW_SUM_FAITHFUL ? launch_sum_t<4, true, 1>(a, nunits, smem, st)
                                         : launch_sum_t<4, false, 1>(a, nunits, smem, st);
-    return mode == FEW_SUM_FAITHFUL ? launch_sum_t<8, true, 1>(a, nunits, smem, st)
-                                    : launch_sum_t<8, false, 1>(a, nunits, smem, st);
+    return mode == FEW_SUM_FAITHFUL ? launch_sum_t<6, true, 1>(a, nunits, smem, st)
+                                    : launch_sum_t<6, false, 1>(a, nunits, smem, st);
 }
 
 }  // namespace few
