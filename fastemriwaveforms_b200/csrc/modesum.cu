@@ -196,8 +196,8 @@ struct SumSamples {
 // One block of NR rows over all columns.  NR is a compile-time count, so the column
 // loop has no test per row: with one the rows' loads and chains cannot be
 // interleaved, and each row waits for its own shared-memory reads (one year, 3843
-// modes: exact 5.73 ms with the test, 4.22 without; faithful 7.13 and 6.65; 363 modes
-// of 63 rows: 1.09 and 0.88).
+// modes: exact 5.73 ms with the test, 4.20 without; faithful 7.13 and 6.65, 6.54 with
+// neighbouring samples as well; 363 modes of 63 rows: 1.09 and 0.88).
 template <int NR, bool FAITHFUL, int SPT, bool THETA>
 __device__ __forceinline__ void sum_rows(const double2 *__restrict__ wblk, const int *rm, const int *rk, int nlo, int NN,
                                          bool theta, const volatile double *park_ep, const volatile double *park_pp,
@@ -300,9 +300,10 @@ __device__ __forceinline__ void sum_rows_of(int rows, const double2 *wblk, const
 
 // One work unit (samples [lo, hi) of segment seg) of the folded sum; the
 // block's shared memory holds the segment's W rows.  Each thread carries SPT
-// samples (i, i + blockDim, ...) through the key loop together, so every
-// shared-memory read of W feeds SPT samples and the samples' dependency chains
-// interleave.  Phi_theta is used when THETA && a.use_theta; THETA = false
+// neighbouring samples through the key loop together, so every shared-memory read of W
+// feeds SPT samples and the samples' dependency chains interleave; neighbours, and not
+// samples blockDim apart, because then whole warps past the end of a unit leave the
+// loop (faithful, 3843 modes: 6.65 -> 6.54 ms at one year of 1000 knots).  Phi_theta is used when THETA && a.use_theta; THETA = false
 // (no row with k' != 0) drops it and its phasor from the registers at compile
 // time, with the same result as a.use_theta = 0.  Ends with a barrier so the
 // caller may reuse shared memory.
@@ -350,12 +351,13 @@ __device__ __forceinline__ void sum_unit(const SumArgs &a, int seg, int lo, int 
             }
         }
         __syncthreads();
-        for (int ib = lo + threadIdx.x; ib < hi; ib += SPT * blockDim.x) {
+        // a thread's samples are neighbours, so that the warps past a unit's end have none
+        for (int ib = lo + SPT * (int)threadIdx.x; ib < hi; ib += SPT * blockDim.x) {
             SumSamples<SPT> m;
 #pragma unroll
             for (int sm = 0; sm < SPT; ++sm) {
                 // a sample past the end repeats the first one; its result is dropped
-                const int i = (ib + sm * (int)blockDim.x < hi) ? ib + sm * (int)blockDim.x : ib;
+                const int i = ib + sm < hi ? ib + sm : ib;
                 // Sample time and phases exactly as interpolate.cu:626-644.
                 const double t = rmul(a.dt, (double)i);
                 m.x[sm] = rsub(t, t0);
@@ -388,7 +390,7 @@ __device__ __forceinline__ void sum_unit(const SumArgs &a, int seg, int lo, int 
             }
 #pragma unroll
             for (int sm = 0; sm < SPT; ++sm) {
-                const int i = ib + sm * (int)blockDim.x;
+                const int i = ib + sm;
                 if (i < hi) {
                     double2 o = a.wf[i];
                     o.x += m.h[sm].x;
@@ -474,9 +476,9 @@ struct SumShape {
 };
 
 // Measured on B200, one year, 3843 modes (R = 21 rows, NN = 61 columns): faithful 7
-// rows x 2 samples 6.65 ms (6.81 with 6 rows, 7.16 with 5, 7.06 at 8 x 1 and 4 x 1,
-// 7.09 at 4 x 2); exact 6 x 1 4.22 ms (4.18 with 7, 4.33 with 4, 4.33 at 8 x 2), and
-// 0.88 ms on 363 modes with k' != 0 (R = 63, NN = 11; 0.89 with 7).  FP64 pipe 70 %
+// rows x 2 samples 6.54 ms (6.81 with 6 rows, 7.16 with 5, 7.06 at 8 x 1 and 4 x 1,
+// 7.09 at 4 x 2, these before neighbouring samples); exact 6 x 1 4.20 ms (4.18 with 7, 4.33 with 4, 4.33 at 8 x 2,
+// 4.31 at 4 x 1, 4.54 at 3 x 2), and 0.88 ms on 363 modes with k' != 0 (R = 63, NN = 11; 0.89 with 7).  FP64 pipe 70 %
 // busy in the faithful form.  FEW_B200_SUM_SHAPE="RBxSPT" overrides both: 4 rows, or 8
 // for the most that there is.
 SumShape sum_shape(int mode)
