@@ -124,8 +124,9 @@ __device__ __forceinline__ void sincos_phase_core(double ph, double *s, double *
     const double hz = 0.5 * z, w = 1.0 - hz;
     const double cn = w + __fma_rn(z * z, u, (1.0 - w) - hz);
     const double a = (q & 1) ? cn : sn, b = (q & 1) ? sn : cn;
-    *s = (q & 2) ? -a : a;
-    *c = ((q + 1) & 2) ? -b : b;
+    // the quadrant's signs, into the sign bits
+    *s = __hiloint2double(__double2hiint(a) ^ ((q & 2) << 30), __double2loint(a));
+    *c = __hiloint2double(__double2hiint(b) ^ (((q + 1) & 2) << 30), __double2loint(b));
 }
 
 // The same for any angle: larger and non-finite ones go to sincos.

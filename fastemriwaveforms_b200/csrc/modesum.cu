@@ -476,9 +476,10 @@ struct SumShape {
 };
 
 // Measured on B200, one year, 3843 modes (R = 21 rows, NN = 61 columns): faithful 7
-// rows x 2 samples 6.54 ms (6.81 with 6 rows, 7.16 with 5, 7.06 at 8 x 1 and 4 x 1,
-// 7.09 at 4 x 2, these before neighbouring samples); exact 6 x 1 4.20 ms (4.18 with 7, 4.33 with 4, 4.33 at 8 x 2,
-// 4.31 at 4 x 1, 4.54 at 3 x 2), and 0.88 ms on 363 modes with k' != 0 (R = 63, NN = 11; 0.89 with 7).  FP64 pipe 70 %
+// rows x 2 samples 6.54 ms (before neighbouring samples 6.65; 6.81 with 6 rows, 7.16
+// with 5, 7.06 at 8 x 1 and 4 x 1, 7.09 at 4 x 2); exact 6 x 1 4.20 ms (4.18 with 7,
+// 4.33 with 4, 4.33 at 8 x 2, 4.31 at 4 x 1 and 4.54 at 3 x 2 with neighbours), and
+// 0.88 ms on 363 modes with k' != 0 (R = 63, NN = 11; 0.89 with 7).  FP64 pipe 70 %
 // busy in the faithful form.  FEW_B200_SUM_SHAPE="RBxSPT" overrides both: 4 rows, or 8
 // for the most that there is.
 SumShape sum_shape(int mode)
