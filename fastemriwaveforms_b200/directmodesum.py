@@ -12,7 +12,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .summation import SummationBase, _input, _ptr, _stream, _to_device, _to_host
+from .summation import SummationBase, _input, _ptr, _stream, _to_host, _upload_packed
 
 
 class DirectModeSum(SummationBase):
@@ -40,7 +40,7 @@ class DirectModeSum(SummationBase):
             ph = torch.stack([_input(p, torch.float64, dev).reshape(-1) for p in phases_in]).contiguous()
         if tuple(ph.shape) != (3, N):
             raise ValueError("phases_in must hold (Phi_phi, Phi_theta, Phi_r), each of len(t) values.")
-        l_d, m_d, k_d, n_d = (_to_device(_to_host(v, np.int32), torch.int32, dev) for v in (l_arr, m_arr, k_arr, n_arr))
+        l_d, m_d, k_d, n_d = _upload_packed([_to_host(v, np.int32) for v in (l_arr, m_arr, k_arr, n_arr)], dev)
         out = torch.empty(N, dtype=torch.complex128, device=dev)
         _lib.call("few_direct_sum", _ptr(teuk), _ptr(y), _ptr(ph), _ptr(l_d), _ptr(m_d), _ptr(k_d), _ptr(n_d), N, K,
                   _ptr(out), _stream(dev))
