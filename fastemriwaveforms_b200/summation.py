@@ -97,7 +97,7 @@ def _upload_packed(arrays, device) -> list:
     return [dev[o:o + a.nbytes].view(_TORCH_TYPES[a.dtype]) for a, o in zip(arrays, starts)]
 
 
-_TORCH_TYPES = {np.dtype(np.float64): torch.float64, np.dtype(np.int32): torch.int32}
+_TORCH_TYPES = {np.dtype(np.float64): torch.float64, np.dtype(np.int32): torch.int32, np.dtype(np.int8): torch.int8}
 
 _COPY_STREAMS: dict = {}
 
@@ -636,8 +636,8 @@ class InterpolatedModeSum(SummationBase):
         p.teuk, p.teuk_in, p.pc_in = teuk, (teuk_in if keep else None), (pc_in if keep else None)
         p.seg = _SegmentPlan(h_t, phase_t, self.num_pts, dt, self.chunk, dev)
         # ylms[K:] *= (-1)^l (interpolatedmodesum.py:357-358)
-        sign = np.ones((2, K))
-        sign[1, l_h % 2 != 0] = -1.0
+        sign = np.ones((2, K), np.int8)
+        sign[1, l_h % 2 != 0] = -1
         p.t_dev, p.fac, sign_dev, p.seg.d_seg_info, p.seg.d_units = _upload_packed(
             (h_t, spline_factor_host(h_t), sign, *p.seg.tables()), dev)
         ylm = torch.view_as_real(_input(ylms, torch.complex128, dev).detach().resolve_conj())
