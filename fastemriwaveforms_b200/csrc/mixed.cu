@@ -323,25 +323,31 @@ __device__ void sum_prod_unit(const MixedArgs &a, int seg, int lo, int hi, unsig
     const int ng = NB / 16, gs = (ng + 1) / 2;  // 16-column groups; half 0 takes [0, gs)
     const int g_lo = h ? gs : 0, g_hi = h ? ng : gs;
 
-    for (int base = lo; base < hi; base += kMT) {
+    // What a tile's epilogue needs of its production.
+    struct Tile {
+        double2 o;
+        float2 Ep, Et;
+        float tau;
+        int i;
+    };
+    const auto produce = [&](int base, Tile &tl) {
         const int i = base + row;
-        const bool valid = i < hi;
+        tl.i = i;
         // the output sample, read early (half 0 adds both halves' sums into it)
-        double2 o = make_double2(0.0, 0.0);
-        if (!h && valid) o = a.wf[i];
+        if (!h && i < hi) tl.o = a.wf[i];
         // FP64 prelude: phases (interpolate.cu:626-644) and anchors.  Rows past the
         // unit (and n' past NN, whose B rows are zero) hold finite phasors whose
         // products are discarded or vanish, so nothing is masked.
         const double t = (double)i * a.dt;
-        const float tau = (float)((t - t0) * ihs);
+        tl.tau = (float)((t - t0) * ihs);
         const double sp = (t - pt0) * ipw;
         const double sp1 = 1.0 - sp;
         const double Pr = phase_poly(s.pc + 16, sp, sp1);
         const float2 Er = anchor(Pr);
         const float2 Er2 = fcmul(Er, Er);
         // the epilogue's phasors, ahead of the chunk loop so that their latency is hidden
-        const float2 Ep = anchor(phase_poly(s.pc, sp, sp1));
-        const float2 Et = a.use_theta ? anchor(phase_poly(s.pc + 8, sp, sp1)) : make_float2(1.f, 0.f);
+        tl.Ep = anchor(phase_poly(s.pc, sp, sp1));
+        tl.Et = a.use_theta ? anchor(phase_poly(s.pc + 8, sp, sp1)) : make_float2(1.f, 0.f);
         for (int k = h; k < nch; k += 2) {
             const int b = sum_stage(k, rg.nas);
             const uint32_t pb = (ro.par >> b) & 1u;
@@ -377,6 +383,10 @@ __device__ void sum_prod_unit(const MixedArgs &a, int seg, int lo, int hi, unsig
             ro.par ^= 1u << b;
             ro.used |= 1u << b;
         }
+    };
+    const auto epilogue = [&](const Tile &tl) {
+        const float2 Ep = tl.Ep, Et = tl.Et;
+        const float tau = tl.tau;
         // accumulator of this tile: this thread's row (TMEM lane), half h's column
         // groups; two (m', k') rows of 8 columns per 16-column load, two loads in
         // flight; u_r by one multiplication when m' steps by one
@@ -428,13 +438,25 @@ __device__ void sum_prod_unit(const MixedArgs &a, int seg, int lo, int hi, unsig
         if (lane == 0) mbar_arrive(&s.acce);
         if (h) s.part[ro.tiles & 1u][row] = Sp;
         sum_prod_sync();
-        if (!h && valid && !ro.dead) {
+        if (!h && tl.i < hi && !ro.dead) {
             const float2 o2 = s.part[ro.tiles & 1u][row];
-            o.x += (double)(Sp.x + o2.x);
-            o.y += (double)(Sp.y + o2.y);
-            a.wf[i] = o;
+            a.wf[tl.i] = make_double2(tl.o.x + (double)(Sp.x + o2.x), tl.o.y + (double)(Sp.y + o2.y));
         }
         ro.tiles++;
+    };
+
+    // With a stage for every chunk of a tile the next tile is written before this one's
+    // accumulator is read, under its MMAs.  With fewer stages it must not be: a chunk
+    // that shares a stage with an earlier one waits for that one's MMAs, and these wait
+    // for the accumulator.
+    const bool ahead = nch <= 2 * rg.nas;
+    Tile cur, nxt;
+    for (int base = ahead ? lo - kMT : lo; base < hi; base += kMT) {
+        const int pbase = ahead ? base + kMT : base;
+        cur = nxt;
+        if (pbase < hi) produce(pbase, nxt);
+        if (!ahead) cur = nxt;
+        if (base >= lo) epilogue(cur);
     }
 }
 
@@ -518,18 +540,25 @@ int mixed_dims(int R, int NN, int *NNp, int *NB, int *nchunks, int *tmem_cols)
     return FEW_OK;
 }
 
-// Ring shape of the sum for chunks of NB columns.  By default one A stage per
-// producer half and as many B slots (2..4) as keep two CTAs per SM (<=
-// kTwoCtaBytes of dynamic shared memory): at the one-year 3843-mode workload this
-// measured 0.75 ms against 0.77 ms for two A stages per half with two B slots,
-// and the autotuner's search over both agrees.  nas, nbs > 0 ask for a shape.
+// Ring shape of the sum for chunks of NB columns, nch of them in a tile (0: not known).
+// By default two A stages per producer half where a tile then has a stage for every
+// chunk and is written ahead (3 or 4 chunks; up to 2 they need one), unless that costs
+// the second CTA of an SM; else one; and as many B slots (2..4) as keep two CTAs per SM
+// (<= kTwoCtaBytes of dynamic shared memory).  One year, 3843 modes (4 chunks): 713 us
+// against 741 with one stage; 500 knots, 1000 modes, 1000000 samples 215 and 236; twelve
+// waveforms in the persistent form 2.84 and 4.82 ms.  Not kept: the persistent form for
+// one waveform (778 us; one unit per CTA is scheduled as CTAs end), polls without the
+// timer's read between them (828), tries that suspend for longer (757).  nas, nbs > 0
+// ask for a shape.
 constexpr int kTwoCtaBytes = 112 * 1024;
 size_t mixed_smem_bytes(const SumRing &rg) { return (size_t)2 * rg.nas * kAStage + (size_t)rg.nbs * rg.bslot; }
-SumRing mixed_ring(int NB, int nbs = 0, int nas = 0)
+SumRing mixed_ring(int NB, int nch, int nbs = 0, int nas = 0)
 {
     SumRing rg;
     rg.bslot = 2 * NB * kKC * 2;
-    rg.nas = nas > 0 ? nas : 1;
+    const bool one_cta = NB > 256;  // its accumulator takes more than half of TMEM
+    const bool ahead = (nch == 0 || nch == 3 || nch == 4) && (one_cta || 4 * kAStage + 2 * rg.bslot <= kTwoCtaBytes);
+    rg.nas = nas > 0 ? nas : (ahead ? 2 : 1);
     rg.nbs = nbs > 0 ? nbs
                      : std::max(2, std::min(kMaxBSlots, (kTwoCtaBytes - 2 * rg.nas * kAStage) / rg.bslot));
     return rg;
@@ -580,7 +609,7 @@ int launch_sum_mixed(double2 *wf, const void *Bpk, const double *pc, int N, cons
     a.NN = NN;
     a.use_theta = use_theta;
     a.dt = dt;
-    const SumRing rg = mixed_ring(a.NB);
+    const SumRing rg = mixed_ring(a.NB, a.nchunks);
     const size_t smem = mixed_smem_bytes(rg);
     FEW_CUDA_TRY(ensure_smem_attr((const void *)k_sum_mixed, (int)smem));
     k_sum_mixed<<<nunits, kSumThreads, smem, st>>>(a, rg);
@@ -602,7 +631,7 @@ int launch_sum_mixed_batched(const few_wave_desc *descs, const int *units4, int 
         ctas = 2 * sms;
     }
     ctas = std::min(ctas, nunits);
-    const SumRing rg = mixed_ring(NB, bstages, astages);
+    const SumRing rg = mixed_ring(NB, 0, bstages, astages);
     const size_t smem = mixed_smem_bytes(rg);
     if (smem > 220 * 1024)
         return fail(FEW_ERR_SIZE, "few_sum_mixed_batched: %d A stages per half and %d B stages of %d bytes exceed "
