@@ -684,16 +684,15 @@ def bench_fd(dev, steps: int, fp64_tflops: float, cpu: bool):
              "e2e": {"ms": ems, "value": bins / (ems * 1e-3), "unit": "mode-bins/s", "h2d_bytes_per_step": int(h2d),
                      "d2h_bytes_per_step": int(h.numel() * 16)},
              "fp64_peak_tflops": fp64_tflops}
-    # FP64 work per (mode, bin) evaluation from an ncu capture of k_fd_sum on the one-year
-    # trajectory (DFMA x 2 + DADD + DMUL per bin visited)
-    flops_per_bin = 786.0
+    # algorithmic FP64 work per (mode, bin): the cubic's root, the amplitude, phase and
+    # frequency-derivative polynomials there, the SPA factor and one phasor
+    flops_per_bin = 200.0
     entry["roofline"] = {"bound": "fp64", "kernel": "k_fd_sum", "achieved": bins * flops_per_bin / (kms * 1e-3) / 1e12,
                          "peak": fp64_tflops, "unit": "TFLOP/s",
                          "frac": bins * flops_per_bin / (kms * 1e-3) / 1e12 / fp64_tflops,
                          "peak_source": "measured in this run: few_probe_fp64_fma (FP64 FMA pipe)",
-                         "algorithmic": f"{flops_per_bin:.0f} FP64 flop per (mode, bin) evaluation (ncu count) x {bins}",
-                         "traffic": {"bytes_per_launch_300_modes": 70.5e6,
-                                     "source": "ncu capture of k_fd_sum, first 300 modes of the one-year case"}}
+                         "algorithmic": f"{flops_per_bin:.0f} FP64 flop per (mode, bin) evaluation x {bins}",
+                         "traffic": None}
     if cpu:
         from oracle import oracle as O
 
@@ -757,13 +756,14 @@ def bench_aak(dev, steps: int, cpu: bool, fp64_tflops: float | None = None):
              "ms": ms, "value": L / (ms * 1e-3), "unit": "samples/s",
              "harmonic_value": L * inp.nmodes / (ms * 1e-3)}
     if fp64_tflops:
-        # FP64 work per sample at 18 harmonics from an ncu capture of k_aak (one-year case)
-        flops_per_sample = 8792.0
+        # algorithmic FP64 work per sample: the orbit and its geometry, and per harmonic a
+        # phasor and three amplitudes
+        flops_per_sample = 400.0 + 100.0 * inp.nmodes
         ach = L * flops_per_sample / (ms * 1e-3) / 1e12
         entry["roofline"] = {"bound": "fp64", "kernel": "k_aak", "achieved": ach, "peak": fp64_tflops,
                              "unit": "TFLOP/s", "frac": ach / fp64_tflops,
                              "peak_source": "measured in this run: few_probe_fp64_fma (FP64 FMA pipe)",
-                             "algorithmic": f"{flops_per_sample:.0f} FP64 flop per sample (ncu count, 18 harmonics)"}
+                             "algorithmic": f"{flops_per_sample:.0f} FP64 flop per sample ({inp.nmodes} harmonics)"}
     if cpu:
         from oracle import oracle as O
 
@@ -1171,7 +1171,7 @@ def main():
                 "peak_source": "measured in this run: few_probe_fp64_fma (FP64 FMA pipe)",
                 "algorithmic": f"{flops_per_key_sample} flop x {keys} keys x {T} samples per launch",
                 "launch_ms": stage["sum"]}
-    spline_roof = {"bound": "hbm", "kernel": "k_spline_chunks", "achieved": spline_bytes / (stage["spline"] * 1e-3) / 1e9,
+    spline_roof = {"bound": "hbm", "kernel": "k_spline_build_factored<false>", "achieved": spline_bytes / (stage["spline"] * 1e-3) / 1e9,
                    "peak": pk["hbm_gbs"], "unit": "GB/s",
                    "frac": spline_bytes / (stage["spline"] * 1e-3) / 1e9 / pk["hbm_gbs"],
                    "peak_source": f"{pk_kind} hbm_gbs", "algorithmic": "16 B per (knot, series)",

@@ -894,9 +894,10 @@ __device__ __forceinline__ void fd_bins(const SumArgs &A, const Entry &E, const 
 // takes the general path.
 // Bound by the FP64 pipe's latency and the shared-memory reads together (FP64
 // pipe 48 % busy, issue slots 59 % at 16 warps per SM).  One year, 3843 modes,
-// 889 million (mode, bin) evaluations: 14.75 ms (15.0 with the quadrant's signs by negation and selection); 65.7 ms with every bin on the
-// general path (1390 instructions a bin against about 320), 17.2 ms with one bin
-// a lane, 26.1 ms at 8 warps per SM.
+// 889 million (mode, bin) evaluations: 14.75 ms (15.0 with the quadrant's signs by
+// negation and selection); 65.7 ms with every bin on the general path (1390
+// instructions a bin against about 320), 17.2 ms with one bin a lane, 26.1 ms at 8
+// warps per SM.
 template <int MINB>
 __global__ void __launch_bounds__(kSumThreads, MINB) k_fd_sum(const __grid_constant__ SumArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];

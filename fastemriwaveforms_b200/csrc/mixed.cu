@@ -25,9 +25,10 @@
 // (LBO) and 256 B between 8-row groups (SBO).  A CTA of 8 producer warps and one
 // MMA warp owns a work unit (<= 1024 samples of one segment) at a time, in
 // 128-sample tiles; two producer threads share a sample row.  K runs in chunks
-// of 32 (16 n' x {Re, Im}) through a two-stage ring: the producer half h writes
-// the A chunks k = h, h + 2, ... into stage h while the MMA warp brings each
-// chunk's B into its stage with one bulk copy and issues its MMAs (2 K-steps x
+// of 32 (16 n' x {Re, Im}) through a ring: the producer half h writes the A
+// chunks k = h, h + 2, ... into its one or two stages, the next tile's ahead of
+// this tile's epilogue where every chunk has a stage, while the MMA warp brings each
+// chunk's B into its slot with one bulk copy and issues its MMAs (2 K-steps x
 // 3 split products per group of <= 256 columns); mbarriers gate every hand-off
 // (details at the kernels).  Every wait is bounded and a timeout sets an error
 // word and ends the kernel, freeing TMEM only once the MMAs have drained.
