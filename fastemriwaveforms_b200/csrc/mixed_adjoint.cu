@@ -107,32 +107,33 @@ __device__ __forceinline__ void g_group(const AdjGMixedArgs &a, int gi, int nA, 
                                         const GPrelude &pr, double scaleB, const int *s_rm, const int *s_rk,
                                         unsigned char *aBuf, unsigned char *bBuf)
 {
-    const int R = a.R, NN = a.NN, CB = a.CB, ncb = a.ncb;
+    const int R = a.R, CB = a.CB, ncb = a.ncb;
     const int planeB = a.NB * 64;
     const int k0 = 16 * (lane >> 3) + (lane & 7);  // K row of part 0 (part 1: +8)
     if (gi < nA) {
         // A: tau^c_a v_{n'} for 16 n' and one c_a (MN 64 c_a + 16 blk ..): whole
         // 16-byte MN chunks for both parts
         const int blk = gi >> 1, ca = gi & 1;
-        const int n0 = nrow0 + 16 * blk;
         double2 v = cmul(pr.v0, cpow_int(pr.Er8, 2 * blk));
-        const double f = ca ? pr.tau : 1.0;
+        // tau^c_a goes into the scale: two products and two selections a value less, 1094 ->
+        // 1051 us with the mask gone (1000 modes x 1000000 samples); the same 1.178e-8 from FP64
+        const double scaleA = ca ? kScaleA * pr.tau : kScaleA;
         uint32_t w[2][kDigits][4];  // [part][digit][word]
 #pragma unroll
         for (int qb = 0; qb < 4; ++qb) {
             double re[4], im[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const bool ok = n0 + 4 * qb + e < NN;
-                re[e] = ok ? f * v.x : 0.0;
-                im[e] = ok ? f * v.y : 0.0;
+                // rows past NN feed accumulator rows that nothing reads: not masked
+                re[e] = v.x;
+                im[e] = v.y;
                 v = cmul(v, pr.Er);
             }
             uint32_t t4[kDigits];
-            digit_words(re, kScaleA, t4);
+            digit_words(re, scaleA, t4);
 #pragma unroll
             for (int p = 0; p < kDigits; ++p) w[0][p][qb] = t4[p];
-            digit_words(im, kScaleA, t4);
+            digit_words(im, scaleA, t4);
 #pragma unroll
             for (int p = 0; p < kDigits; ++p) w[1][p][qb] = t4[p];
         }
