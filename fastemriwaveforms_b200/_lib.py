@@ -60,6 +60,7 @@ SIGNATURES = {
     "few_spline_adjoint_factored": [_vp, _vp, _vp, _c_ll, _c_ll, _c_int, _c_ll, _c_int, _c_int, _c_int, _vp],
     "few_spline_adjoint": [_vp, _c_ll, _vp, _vp, _c_ll, _c_ll, _c_int, _c_ll, _c_int, _c_int, _c_int, _vp],
     "few_mixed_operand_bytes": [_c_int, _c_int, _c_int],
+    "few_mixed_ring": [_c_int, _c_int, _c_int, _c_int, _vp],
     "few_fold_mixed": [_vp, _vp, _c_int, _c_int, _c_int, _vp, _vp],
     "few_sum_mixed": [_vp, _vp, _vp, _c_int, _vp, _vp, _vp, _c_int, _vp, _vp, _c_int, _c_int, _c_int, _c_dbl, _c_int,
                       _vp, _vp],

@@ -150,6 +150,14 @@ struct SumShared {
     float2 part[2][kMT];  // half 1's epilogue sums, by tile parity
 };
 
+// Dynamic shared memory of a CTA: at most kRingBytes, and at most kTwoCtaBytes where two
+// CTAs are to share an SM, whose 228 KB also hold each CTA's static part and 1 KB that
+// the driver reserves for it.
+constexpr int kStaticBytes = 3 * 1024;  // SumShared before the 1 KB alignment of the ring
+static_assert(sizeof(SumShared) <= kStaticBytes && sizeof(SumShared) > kStaticBytes - 1024, "static shared memory");
+constexpr int kRingBytes = 220 * 1024;
+constexpr int kTwoCtaBytes = (228 * 1024 - 2 * (1024 + kStaticBytes)) / 2;
+
 // Ring layout of the dynamic shared memory: 2 nas A stages, then nbs B slots.
 struct SumRing {
     int nas;       // A stages per producer half (1 or 2)
@@ -544,21 +552,23 @@ int mixed_dims(int R, int NN, int *NNp, int *NB, int *nchunks, int *tmem_cols)
 // Ring shape of the sum for chunks of NB columns, nch of them in a tile (0: not known).
 // By default two A stages per producer half where a tile then has a stage for every
 // chunk and is written ahead (3 or 4 chunks; up to 2 they need one), unless that costs
-// the second CTA of an SM; else one; and as many B slots (2..4) as keep two CTAs per SM
-// (<= kTwoCtaBytes of dynamic shared memory).  One year, 3843 modes (4 chunks): 713 us
-// against 741 with one stage; 500 knots, 1000 modes, 1000000 samples 215 and 236; twelve
-// waveforms in the persistent form 2.84 and 4.82 ms.  Not kept: the persistent form for
-// one waveform (778 us; one unit per CTA is scheduled as CTAs end), polls without the
-// timer's read between them (828), tries that suspend for longer (757).  nas, nbs > 0
-// ask for a shape.
-constexpr int kTwoCtaBytes = 112 * 1024;
+// the second CTA of an SM; else one; and as many B slots (2..4) as keep two CTAs per SM.
+// The second CTA is worth more than any stage: 500 knots, 1000000 samples, 61 columns,
+// us a call with a two-stage ring that leaves a single CTA and as chosen here: 11 rows
+// 435 and 300, 15 rows 449 and 314, 23 rows 504 and 370 (one stage).
+// One year, 3843 modes (21 rows, 4 chunks): 713 us against 741 with one stage; 500
+// knots, 1000 modes, 1000000 samples 215 and 236; twelve waveforms in the persistent
+// form 2.84 and 4.82 ms.  Not kept: the persistent form for one waveform (778 us; one
+// unit per CTA is scheduled as CTAs end), polls without the timer's read between them
+// (828), tries that suspend for longer (757).  nas, nbs > 0 ask for a shape.
 size_t mixed_smem_bytes(const SumRing &rg) { return (size_t)2 * rg.nas * kAStage + (size_t)rg.nbs * rg.bslot; }
 SumRing mixed_ring(int NB, int nch, int nbs = 0, int nas = 0)
 {
     SumRing rg;
     rg.bslot = 2 * NB * kKC * 2;
     const bool one_cta = NB > 256;  // its accumulator takes more than half of TMEM
-    const bool ahead = (nch == 0 || nch == 3 || nch == 4) && (one_cta || 4 * kAStage + 2 * rg.bslot <= kTwoCtaBytes);
+    const int ahead_bytes = 4 * kAStage + 2 * rg.bslot;
+    const bool ahead = (nch == 0 || nch == 3 || nch == 4) && ahead_bytes <= (one_cta ? kRingBytes : kTwoCtaBytes);
     rg.nas = nas > 0 ? nas : (ahead ? 2 : 1);
     rg.nbs = nbs > 0 ? nbs
                      : std::max(2, std::min(kMaxBSlots, (kTwoCtaBytes - 2 * rg.nas * kAStage) / rg.bslot));
@@ -634,7 +644,7 @@ int launch_sum_mixed_batched(const few_wave_desc *descs, const int *units4, int 
     ctas = std::min(ctas, nunits);
     const SumRing rg = mixed_ring(NB, 0, bstages, astages);
     const size_t smem = mixed_smem_bytes(rg);
-    if (smem > 220 * 1024)
+    if (smem > kRingBytes)
         return fail(FEW_ERR_SIZE, "few_sum_mixed_batched: %d A stages per half and %d B stages of %d bytes exceed "
                     "shared memory", rg.nas, rg.nbs, rg.bslot);
     FEW_CUDA_TRY(ensure_smem_attr((const void *)k_sum_mixed_batched, (int)smem));
@@ -667,6 +677,23 @@ extern "C" int few_fold_mixed(const void *W, const double *t_knots, int nseg, in
     if (!W || !t_knots || !Bpk) return few::fail(FEW_ERR_ARG, "few_fold_mixed: null pointer");
     if (nseg < 0 || R < 1 || NN < 1) return few::fail(FEW_ERR_SIZE, "few_fold_mixed: bad sizes");
     return few::launch_fold_mixed((const double2 *)W, t_knots, nseg, R, NN, Bpk, (cudaStream_t)stream);
+}
+
+extern "C" int few_mixed_ring(int R, int nchunks, int astages, int bstages, int *shape)
+{
+    few::clear_error();
+    if (!shape) return few::fail(FEW_ERR_ARG, "few_mixed_ring: null pointer");
+    if (R < 1 || R > few::kMixedMaxRows || nchunks < 0) return few::fail(FEW_ERR_SIZE, "few_mixed_ring: bad sizes");
+    int NNp, NB, nch, cols;
+    int rc = few::mixed_dims(R, 16, &NNp, &NB, &nch, &cols);
+    if (rc) return rc;
+    const few::SumRing rg = few::mixed_ring(NB, nchunks, bstages, astages);
+    shape[0] = rg.nas;
+    shape[1] = rg.nbs;
+    shape[2] = (int)few::mixed_smem_bytes(rg);
+    shape[3] = few::kStaticBytes;
+    shape[4] = cols;
+    return FEW_OK;
 }
 
 extern "C" long long few_mixed_operand_bytes(int nseg, int R, int NN)

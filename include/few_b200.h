@@ -303,15 +303,22 @@ FEW_API int few_sum_mixed(void *wf, const void *Bpk, const double *phase_coeffs,
                           const double *t_knots, const int *units, int nunits, const int *row_m, const int *row_k,
                           int R, int nlo, int NN, double dt, int use_theta, int *err, void *stream);
 
+/* The operand ring that the tensor-core sum takes for R rows and tiles of nchunks chunks
+ * (16 n' each; 0: not known, as in the persistent form), astages and bstages as in
+ * few_sum_mixed_batched (0: the library's choice): shape [host] (5,) = {A stages per
+ * producer half, B slots, dynamic and static bytes of shared memory of a CTA, TMEM
+ * columns of a CTA}.  Makes no CUDA call. */
+FEW_API int few_mixed_ring(int R, int nchunks, int astages, int bstages, int *shape);
+
 /* Persistent form of few_sum_mixed over many waveforms: descs [device]
  * (nwave,) with Bpk set (few_fold_mixed per waveform); units4 [device]
  * (4*nunits,) = {waveform, segment, first sample, end sample}; max_R: the
  * largest R in the batch (<= 64, sizes shared memory and TMEM); ctas:
  * persistent CTAs (0: two per SM); astages: A-operand stages per producer half
  * (1 or 2; 0: 2 where two CTAs per SM still fit, else 1); bstages: depth of the
- * B-operand ring, 2..4 bulk-copy slots
- * (0: as many as keep two CTAs per SM); err [device] int as in few_sum_mixed;
- * done as in few_sum_batched.  Results do not depend on the stage counts. */
+ * B-operand ring, 2..4 bulk-copy slots (0: as many as keep two CTAs per SM; see
+ * few_mixed_ring); err [device] int as in few_sum_mixed; done as in
+ * few_sum_batched.  Results do not depend on the stage counts. */
 FEW_API int few_sum_mixed_batched(const few_wave_desc *descs, int nwave, const int *units4, int nunits, int max_R,
                                   int ctas, int astages, int bstages, int *err, unsigned long long *done,
                                   void *stream);
