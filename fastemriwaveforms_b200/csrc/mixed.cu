@@ -567,7 +567,7 @@ SumRing mixed_ring(int NB, int nch, int nbs = 0, int nas = 0)
     SumRing rg;
     rg.bslot = 2 * NB * kKC * 2;
     const bool one_cta = NB > 256;  // its accumulator takes more than half of TMEM
-    const int ahead_bytes = 4 * kAStage + 2 * rg.bslot;
+    const int ahead_bytes = 4 * kAStage + (nbs > 0 ? nbs : 2) * rg.bslot;
     const bool ahead = (nch == 0 || nch == 3 || nch == 4) && ahead_bytes <= (one_cta ? kRingBytes : kTwoCtaBytes);
     rg.nas = nas > 0 ? nas : (ahead ? 2 : 1);
     rg.nbs = nbs > 0 ? nbs

@@ -1,8 +1,7 @@
 """The operand ring of the tensor-core sum, a host rule (no GPU): two CTAs share an SM
 wherever the accumulators and some ring of at least one A stage and two B slots let
 them; a second A stage is taken only beside the second CTA; an asked shape is kept, and
-one part of it never makes the other too large; and the autotuner's keys name the form
-of the kernels they were timed on."""
+one part of it never makes the other too large."""
 import numpy as np
 import pytest
 
@@ -43,3 +42,17 @@ def test_two_ctas_share_an_sm(nchunks):
         assert nas == (2 if ahead else 1), (R, nchunks)
         if nbs < 4:  # no slot was left out that would have fitted
             assert not two_fit(dyn + b_slot(R), static), (R, nchunks)
+
+
+def test_an_asked_shape_is_kept_and_one_part_leaves_room_for_the_other():
+    for R in range(1, 65):
+        for nchunks in range(6):
+            for bstages in (2, 3, 4):
+                for astages in (1, 2):
+                    assert ring(R, nchunks, astages, bstages)[:2] == (astages, bstages)
+                nas, nbs, dyn, _, _ = ring(R, nchunks, 0, bstages)
+                assert nbs == bstages
+                if ring(R, nchunks, 1, bstages)[2] <= MAX_DYNAMIC:
+                    assert dyn <= MAX_DYNAMIC, (R, nchunks, bstages)
+            for astages in (1, 2):
+                assert ring(R, nchunks, astages, 0)[0] == astages
