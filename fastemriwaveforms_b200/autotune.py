@@ -10,7 +10,7 @@ pipelines hide more latency but take shared memory that a second CTA per SM
 needs.  Each candidate is timed with CUDA events on
 the caller's real batch (the sum kernel only; the rest of the forward does not
 depend on the choice) and the fastest is cached in a JSON file keyed by GPU
-name, precision and the batch's shape buckets.
+name, precision, the batch's shape buckets and the form of the kernels.
 
 Cache location: $FEW_B200_TUNE_CACHE, else ~/.cache/fastemriwaveforms_b200/tune.json.
 """
@@ -64,10 +64,16 @@ def bucket(x: float) -> int:
     return 1 << max(0, int(math.ceil(math.log2(max(x, 1.0)))))
 
 
+# Form of the kernels that are tuned, part of every key: a choice timed on another form is
+# not looked up.  Goes up with each change of k_sum_mixed_batched or k_sum_folded_batched
+# that can move the best shape.
+KERNEL_FORM = 2
+
+
 def key_of(device, precision: str, max_R: int, max_NN: int, mean_seg_len: float, n_wave: int) -> str:
     name = torch.cuda.get_device_name(device).replace(" ", "_")
     return (f"{name}|{precision}|R{bucket(max_R)}|NN{bucket(max_NN)}|L{bucket(mean_seg_len)}"
-            f"|W{bucket(n_wave)}")
+            f"|W{bucket(n_wave)}|v{KERNEL_FORM}")
 
 
 def lookup(key: str):

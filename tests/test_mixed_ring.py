@@ -1,11 +1,12 @@
 """The operand ring of the tensor-core sum, a host rule (no GPU): two CTAs share an SM
 wherever the accumulators and some ring of at least one A stage and two B slots let
 them; a second A stage is taken only beside the second CTA; an asked shape is kept, and
-one part of it never makes the other too large."""
+one part of it never makes the other too large; and the autotuner's keys name the form
+of the kernels they were timed on."""
 import numpy as np
 import pytest
 
-from fastemriwaveforms_b200 import _lib
+from fastemriwaveforms_b200 import _lib, autotune
 
 SM_SHARED = 228 * 1024   # shared memory of an SM (sm_100)
 RESERVED = 1024          # per resident CTA, by the driver
@@ -56,3 +57,11 @@ def test_an_asked_shape_is_kept_and_one_part_leaves_room_for_the_other():
                     assert dyn <= MAX_DYNAMIC, (R, nchunks, bstages)
             for astages in (1, 2):
                 assert ring(R, nchunks, astages, 0)[0] == astages
+
+
+def test_tuned_choices_belong_to_the_form_of_the_kernels(monkeypatch):
+    monkeypatch.setattr(autotune.torch.cuda, "get_device_name", lambda device: "B200")
+    key = autotune.key_of(None, "mixed", 21, 61, 3000.0, 12)
+    assert key.endswith(f"|v{autotune.KERNEL_FORM}")
+    monkeypatch.setattr(autotune, "KERNEL_FORM", autotune.KERNEL_FORM + 1)
+    assert autotune.key_of(None, "mixed", 21, 61, 3000.0, 12) != key
