@@ -112,6 +112,9 @@ class BatchedInterpolatedModeSum:
         max_NN = max(p.fold.NN for p in self.preps)
         if self.precision == "mixed" and self.max_R > 64:
             raise ValueError("precision='mixed' supports at most 64 (m, k) rows")
+        if self.precision != "mixed" and max_NN * 64 > 200 * 1024:
+            raise ValueError(f"the FP64 sum holds at least one (m, k) row in shared memory: {max_NN} values of n exceed "
+                             "the 3200 that fit")
         # the FP64 kernels keep a segment's rows in shared memory in blocks of up to 8 rows
         self.smem_bytes = int(min(200 * 1024, max((p.fold.R + 7) // 8 * 8 * p.fold.NN * 64 for p in self.preps)))
         descs = np.zeros(len(self.preps), DESC_DTYPE)

@@ -168,22 +168,29 @@ struct SumArgs {
     const int *row_m;
     const int *row_k;
     int N, R, nlo, NN;
-    int blocks_per_pass;  // row blocks whose coefficients are in shared memory at once
+    int nblk;             // row blocks
+    int blocks_per_pass;  // of them, those whose coefficients are in shared memory at once
     int use_theta;
     double dt;
 };
 
-// The rows go through the registers in ceil(R / RB) blocks of nearly equal size (RB
-// rows at most); block b starts at row row_block(b).
-__host__ __device__ inline int row_blocks(int R, int RB) { return (R + RB - 1) / RB; }
+// The rows go through the registers in nblk blocks of nearly equal size (RB rows at
+// most, and no more than shared memory holds); block b starts at row row_block(b).
 __host__ __device__ inline int row_block(int b, int R, int nblk) { return (int)((long long)b * R / nblk); }
 
-// Blocks per pass: all when their coefficients fit in smem_bytes, else the most that
-// surely fit (0 if not even one does).
-__host__ __device__ inline int sum_blocks_per_pass(int R, int NN, int RB, int smem_bytes)
+// Row blocks of a sum, and how many go through shared memory in a pass: all when their
+// coefficients fit in smem_bytes, else the most that surely fit.  None of either when
+// not even one row's do.
+struct SumBlocks {
+    int nblk, per_pass;
+};
+
+__host__ __device__ inline SumBlocks sum_blocks(int R, int NN, int RB, int smem_bytes)
 {
-    const int nblk = row_blocks(R, RB), fit = smem_bytes / (NN * 4 * (int)sizeof(double2));  // rows that fit
-    return R <= fit ? nblk : fit / ((R + nblk - 1) / nblk);
+    const int fit = (int)(smem_bytes / (NN * 4LL * (long long)sizeof(double2)));  // rows that fit
+    if (fit < 1) return SumBlocks{0, 0};
+    const int most = RB < fit ? RB : fit, nblk = (R + most - 1) / most;
+    return SumBlocks{nblk, R <= fit ? nblk : fit / ((R + nblk - 1) / nblk)};
 }
 
 // A thread's samples between row blocks.
@@ -312,7 +319,7 @@ __device__ __forceinline__ void sum_unit(const SumArgs &a, int seg, int lo, int 
                                          double *s_pc)
 {
     const double t0 = a.seg_info[3 * seg], pt0 = a.seg_info[3 * seg + 1], pw = a.seg_info[3 * seg + 2];
-    const int R = a.R, NN = a.NN, nlo = a.nlo, nblk = row_blocks(R, RB);
+    const int R = a.R, NN = a.NN, nlo = a.nlo, nblk = a.nblk;
     const long long nps = (long long)(a.N - 1) * 3;
     const bool theta = THETA && a.use_theta;
     // The faithful form parks Phi_phi and e^{-i Phi_phi}, needed only at each
@@ -444,7 +451,9 @@ __global__ void __launch_bounds__(kSumThreads, (SPT == 1 || RB <= 4) ? 2 : 1) k_
         a.NN = d.NN;
         a.use_theta = d.use_theta;
         a.dt = d.dt;
-        a.blocks_per_pass = sum_blocks_per_pass(d.R, d.NN, RB, smem_bytes);
+        const SumBlocks sb = sum_blocks(d.R, d.NN, RB, smem_bytes);
+        a.nblk = sb.nblk;
+        a.blocks_per_pass = sb.per_pass;
         sum_unit<RB, FAITHFUL, SPT, true>(a, units4[4 * u + 1], units4[4 * u + 2], units4[4 * u + 3],
                                     reinterpret_cast<double2 *>(smem_raw), s_rm, s_rk, s_pc);
         if (done) {  // completion time of the waveform: the latest of its units
@@ -574,11 +583,11 @@ int launch_sum_folded(double2 *wf, const double2 *W, const double *pc, int N, co
     a.dt = dt;
     const long long row_bytes = (long long)NN * 4 * sizeof(double2);
     const SumShape sh = sum_shape(mode);
-    const int nblk = row_blocks(R, sh.rb), bpp = sum_blocks_per_pass(R, NN, sh.rb, kSmemBudget);
-    if (bpp < 1)
-        return fail(FEW_ERR_SIZE, "few_sum_folded: NN=%d too large for one row block in shared memory", NN);
-    a.blocks_per_pass = bpp;
-    const size_t smem = (size_t)std::min(R, bpp * ((R + nblk - 1) / nblk)) * row_bytes;
+    const SumBlocks sb = sum_blocks(R, NN, sh.rb, kSmemBudget);
+    if (sb.nblk < 1) return fail(FEW_ERR_SIZE, "few_sum_folded: NN=%d too large for one row in shared memory", NN);
+    a.nblk = sb.nblk;
+    a.blocks_per_pass = sb.per_pass;
+    const size_t smem = (size_t)std::min(R, sb.per_pass * ((R + sb.nblk - 1) / sb.nblk)) * row_bytes;
     if (sh.rb == 4 && sh.spt == 2)
         return mode == FEW_SUM_FAITHFUL ? launch_sum_t<4, true, 2>(a, nunits, smem, st)
                                         : launch_sum_t<4, false, 2>(a, nunits, smem, st);
@@ -622,6 +631,19 @@ extern "C" int few_fold_slopes(const void *y, const void *slopes, const double *
         (const double2 *)y, (const double2 *)slopes, fac, (const double2 *)ylms, key_ptr, key_list, K, nseg, nkeys,
         (double2 *)W);
     FEW_LAUNCH_CHECK("k_fold_slopes");
+    return FEW_OK;
+}
+
+extern "C" int few_sum_row_blocks(int R, int NN, int smem_bytes, int mode, int *blocks)
+{
+    few::clear_error();
+    if (!blocks) return few::fail(FEW_ERR_ARG, "few_sum_row_blocks: null pointer");
+    if (R < 1 || R > few::kMaxRows || NN < 1 || smem_bytes < 1 || smem_bytes > few::kSmemBudget)
+        return few::fail(FEW_ERR_SIZE, "few_sum_row_blocks: bad sizes");
+    if (mode != FEW_SUM_FAITHFUL && mode != FEW_SUM_EXACT) return few::fail(FEW_ERR_ARG, "few_sum_row_blocks: bad mode");
+    const few::SumBlocks sb = few::sum_blocks(R, NN, few::sum_shape(mode).rb, smem_bytes);
+    blocks[0] = sb.nblk;
+    blocks[1] = sb.per_pass;
     return FEW_OK;
 }
 

@@ -259,12 +259,20 @@ FEW_API int few_sum_folded(void *wf, const void *W, const double *phase_coeffs, 
                    const int *units, int nunits, const int *row_m, const int *row_k, int R, int nlo,
                    int NN, double dt, int mode, int use_theta, void *stream);
 
+/* How the sum takes R rows of NN columns with smem_bytes (<= 200 KiB) of shared memory
+ * for their coefficients: blocks [host] (2,) = {blocks of nearly equal numbers of rows,
+ * blocks per pass over the samples}; zeros when one row does not fit (NN > 3200 at 200
+ * KiB; few_sum_folded refuses these).  Makes no CUDA call. */
+FEW_API int few_sum_row_blocks(int R, int NN, int smem_bytes, int mode, int *blocks);
+
 /* Persistent form of few_sum_folded over many waveforms (no counterpart in
  * the reference, which launches one kernel per knot segment of one waveform):
  * descs [device] (nwave,); units4 [device] (4*nunits,) = {waveform, segment,
  * first sample, end sample}, segments' samples as few_segment_plan makes
  * them (units of one waveform must not overlap).  smem_bytes: dynamic shared
- * memory per CTA (<= 200 KiB; the largest R*NN*64 of the batch, capped);
+ * memory per CTA (<= 200 KiB; the largest R*NN*64 of the batch, capped): a
+ * waveform of which not even one row's NN*64 bytes fit (see few_sum_row_blocks)
+ * is left out;
  * ctas: persistent CTAs (0: two per SM).  mode FEW_SUM_FAITHFUL or FEW_SUM_EXACT.
  * done [device] (nwave,) or NULL: each waveform's completion time, the
  * %globaltimer nanoseconds after its last work unit, merged with atomicMax
