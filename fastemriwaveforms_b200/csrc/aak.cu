@@ -18,10 +18,15 @@
 //   * Amplitudes.  The three Bessel combinations of a harmonic depend on e alone,
 //     and e hardly moves over the few hundred samples of a CTA: they are computed
 //     at 6, 8 or 12 Chebyshev nodes of the CTA's own range of e (the fewest whose
-//     interpolation error stays below 1e-17) and evaluated as polynomials there.
+//     truncation error stays below 1e-17) and evaluated as polynomials there.
 //     At a node the five Bessel values of a harmonic come from one backward
-//     (Miller) recurrence normalised by J_0 + 2 sum J_2k = 1.  Where e moves too
-//     far for 12 nodes, every sample runs the recurrence.
+//     (Miller) recurrence normalised by J_0 + 2 sum J_2k = 1, moved to the node's
+//     exact argument.  Where e moves too far for 12 nodes, every sample runs the
+//     recurrence.  Rounding: against long double on a CPU, over e = 0.2-0.65 and
+//     up to 40 harmonics, the strong harmonics (above 1e-3) are off by 2.8, 3.7
+//     and 3.7e-16 of their largest value (rms; at most 1.7, 2.6 and 2.6e-15) with
+//     6, 8 and 12 nodes; by the recurrence alone 4.6, 4.5 and 5.0e-16 (3.2, 3.3
+//     and 4.8e-15) over the same ranges.
 //   * Phases.  e^{i n Phi} by a running product of e^{i Phi}; the reference rounds
 //     n Phi (+ Doppler), at phases of ~1e7 rad, and that rounding is part of the
 //     result: its exact error eps (|eps| < 4e-9) comes from error-free
@@ -199,9 +204,17 @@ __device__ __forceinline__ void cross3(const double *u, const double *v, double 
 }
 
 // ---- Chebyshev interpolation on Q nodes ------------------------------------------
-// node[j] = cos((j + 1/2) pi / Q); v[k][j]: the coefficient of u^k of the interpolant
-// is sum_j v[k][j] f(node_j) (the discrete Chebyshev coefficients, then T_m by
-// powers of u).
+// node[j] = cos((j + 1/2) pi / Q); sum_j d[m][j] f(node_j): the coefficient of T_m of
+// the interpolant; t[m][k]: T_m's coefficient of u^k (whole numbers).
+//
+// The interpolant is evaluated by powers of u, whose true coefficients fall off as
+// (n delta)^k / k!, so that Horner's rule loses nothing; the way there must not lose
+// anything either: the T_m's coefficients reach 2^(Q-1) and cancel.  So the
+// coefficients of T_m are formed from differences to one node's value, and the sums
+// over m that turn them into powers of u carry their rounding errors (two-sum and
+// two-product): what a node's value is off by then stays a polynomial of that size
+// (Chebyshev nodes pass it on by a factor of 2 at most, less than 1 on average).  With
+// plain sums 12 nodes are off by up to 3e-13 and 8 by 1e-14.
 constexpr double const_cos(double x) {  // Taylor, 0 <= x <= pi
     const bool flip = x > 1.5707963267948966;
     const double r = flip ? kPi - x : x;
@@ -217,39 +230,68 @@ constexpr int kMaxNodes = 12;
 
 struct Cheb {
     double node[kMaxNodes];
-    double v[kMaxNodes][kMaxNodes];
+    double d[kMaxNodes][kMaxNodes];
+    double t[kMaxNodes][kMaxNodes];
 };
 
 constexpr Cheb make_cheb(int Q) {
     Cheb t{};
-    double T[kMaxNodes][kMaxNodes] = {};  // T_m by powers
-    T[0][0] = 1.0;
-    T[1][1] = 1.0;
+    t.t[0][0] = 1.0;
+    t.t[1][1] = 1.0;
     for (int m = 2; m < Q; ++m)
-        for (int k = 0; k < Q; ++k) T[m][k] = (k > 0 ? 2.0 * T[m - 1][k - 1] : 0.0) - T[m - 2][k];
+        for (int k = 0; k < Q; ++k) t.t[m][k] = (k > 0 ? 2.0 * t.t[m - 1][k - 1] : 0.0) - t.t[m - 2][k];
     for (int j = 0; j < Q; ++j) {
         t.node[j] = const_cos((j + 0.5) * kPi / Q);
         double c[kMaxNodes] = {};  // T_m(node_j)
         c[0] = 1.0;
         c[1] = t.node[j];
         for (int m = 2; m < Q; ++m) c[m] = 2.0 * t.node[j] * c[m - 1] - c[m - 2];
-        for (int k = 0; k < Q; ++k) {
-            double sum = 0.0;
-            for (int m = 0; m < Q; ++m) sum += (m == 0 ? 1.0 : 2.0) / Q * c[m] * T[m][k];
-            t.v[k][j] = sum;
-        }
+        for (int m = 0; m < Q; ++m) t.d[m][j] = (m == 0 ? 1.0 : 2.0) / Q * c[m];
     }
     return t;
 }
 
-__constant__ Cheb c_cheb[3] = {make_cheb(6), make_cheb(8), make_cheb(12)};
+// in global memory: the lanes of a warp read different entries
+__device__ const Cheb c_cheb[3] = {make_cheb(6), make_cheb(8), make_cheb(12)};
 
 constexpr int kThreads = 128;
 constexpr int kHarm = 24;  // harmonics whose polynomials a CTA holds at a time (even: they come in pairs)
 
+// Values at the nodes, co[row * kMaxNodes + j] -> coefficients of the powers of u, in
+// place; by way of cheb[row * (kMaxNodes + 1) + m], the coefficients of T_m, and behind
+// them the value that these are relative to.  One barrier inside.
+template <int Q>
+__device__ __forceinline__ void to_powers(const Cheb &T, int rows, double *co, double *cheb) {
+    for (int w = threadIdx.x; w < rows * Q; w += kThreads) {
+        const int r = w / Q, m = w - r * Q;
+        const double *f = co + r * kMaxNodes;
+        const double ref = f[Q / 2];
+        double sum = 0.0;
+#pragma unroll
+        for (int j = 0; j < Q; ++j) sum = fma(T.d[m][j], f[j] - ref, sum);
+        cheb[r * (kMaxNodes + 1) + m] = sum;
+        if (m == 0) cheb[r * (kMaxNodes + 1) + kMaxNodes] = ref;
+    }
+    __syncthreads();
+    for (int w = threadIdx.x; w < rows * Q; w += kThreads) {
+        const int r = w / Q, k = w - r * Q;
+        const double *a = cheb + r * (kMaxNodes + 1);
+        double hi = 0.0, lo = 0.0;
+#pragma unroll
+        for (int i = 0; i < Q / 2; ++i) {  // m of k's parity; below k T_m has no u^k
+            const int m = 2 * i + (k & 1);
+            const double t = T.t[m][k], p = rmul(t, a[m]), sum = radd(hi, p);
+            lo += two_sum_err(hi, p, sum) + fma(t, a[m], -p);
+            hi = sum;
+        }
+        co[r * kMaxNodes + k] = radd(hi, lo) + (k == 0 ? a[kMaxNodes] : 0.0);
+    }
+}
+
 // Largest n * (half width of the e range) for Q nodes: the interpolant of a
 // function whose Q-th derivative is at most n^Q errs by at most
-// (n delta)^Q / (2^(Q-1) Q!), kept below 1e-17.
+// (n delta)^Q / (2^(Q-1) Q!), kept below 1e-17 (of the sum's scale; a harmonic too
+// weak to matter is truncated at a larger share of itself).
 __device__ __forceinline__ int node_set(double nd) { return nd <= 7.8e-3 ? 0 : (nd <= 0.052 ? 1 : (nd <= 0.38 ? 2 : 3)); }
 
 // The three combinations of harmonic n's Bessel values J_{n-2..n+2}(n e).
@@ -257,6 +299,22 @@ __device__ __forceinline__ void combine(int n, double e, const double J[5], doub
     f[0] = -n * (J[0] - 2. * e * J[1] + 2. / n * J[2] + 2. * e * J[3] - J[4]);
     f[1] = -n * (J[0] - 2. * J[2] + J[4]);
     f[2] = 2. * J[2];
+}
+
+// Bessel values J_{n-2..n+2} that the recurrence gave for x = fl(n e), moved to n e: it
+// worked at 2 / fl(2 / x), an n-th power of whose rounding a value of order n carries
+// (the largest part of its error).  J_k' = J_{k-1} - k/x J_k = k/x J_k - J_{k+1}.
+__device__ __forceinline__ void to_exact_argument(int n, double e, double x, double J[5]) {
+    if (x == 0.0) return;
+    const double tox = 2.0 / x;
+    const double dx = fma(0.5 * fma(tox, x, -2.0), x, fma((double)n, e, -x));
+    const double ix = 0.5 * tox;
+    double d[5];
+    d[0] = (n - 2) * ix * J[0] - J[1];
+#pragma unroll
+    for (int q = 1; q < 5; ++q) d[q] = J[q - 1] - (n - 2 + q) * ix * J[q];
+#pragma unroll
+    for (int q = 0; q < 5; ++q) J[q] = fma(dx, d[q], J[q]);
 }
 
 // Per-launch angles, once per CTA (one sine and cosine a lane).
@@ -336,6 +394,7 @@ template <int P, bool MICH>
 __global__ void __launch_bounds__(kThreads, 4) k_aak(AakArgs A) {
     __shared__ Sky K;
     __shared__ double s_co[kHarm * 3 * kMaxNodes];
+    __shared__ double s_cheb[kHarm * 3 * (kMaxNodes + 1)];  // coefficients of T_m; the value they are relative to
     __shared__ double s_min[kThreads / 32], s_max[kThreads / 32];
     const int tid = threadIdx.x, lane = tid & 31;
     const int i0 = A.first[0], i1 = A.first[A.nseg];
@@ -446,7 +505,10 @@ __global__ void __launch_bounds__(kThreads, 4) k_aak(AakArgs A) {
                 const int pr = w / Q, j = w - pr * Q, n = n0 + 2 * pr;
                 const double en = fma(delta, T.node[j], ec);
                 double Ja[5], Jb[5], f[3];
-                bessel_band2(n, n * en, (n + 1) * en, Ja, Jb);
+                const double xa = n * en, xb = (n + 1) * en;
+                bessel_band2(n, xa, xb, Ja, Jb);
+                to_exact_argument(n, en, xa, Ja);
+                to_exact_argument(n + 1, en, xb, Jb);
                 combine(n, en, Ja, f);
 #pragma unroll
                 for (int q = 0; q < 3; ++q) s_co[(2 * pr * 3 + q) * kMaxNodes + j] = f[q];
@@ -455,19 +517,9 @@ __global__ void __launch_bounds__(kThreads, 4) k_aak(AakArgs A) {
                 for (int q = 0; q < 3; ++q) s_co[((2 * pr + 1) * 3 + q) * kMaxNodes + j] = f[q];
             }
             __syncthreads();
-            // values at the nodes -> coefficients of the powers of u, in place
-            for (int w = tid; w < count * 3; w += kThreads) {
-                double *c = s_co + w * kMaxNodes;
-                double f[kMaxNodes];
-#pragma unroll
-                for (int j = 0; j < kMaxNodes; ++j) f[j] = j < Q ? c[j] : 0.0;
-                for (int k = 0; k < Q; ++k) {
-                    double sum = 0.0;
-#pragma unroll
-                    for (int j = 0; j < kMaxNodes; ++j) sum = fma(T.v[k][j], f[j], sum);
-                    c[k] = sum;
-                }
-            }
+            if (set == 0) to_powers<6>(T, count * 3, s_co, s_cheb);
+            else if (set == 1) to_powers<8>(T, count * 3, s_co, s_cheb);
+            else to_powers<12>(T, count * 3, s_co, s_cheb);
             __syncthreads();
             if (set == 0) H.template table<6>(n0, count, s_co, A, K, cosorb);
             else if (set == 1) H.template table<8>(n0, count, s_co, A, K, cosorb);
