@@ -84,7 +84,9 @@ __global__ void __launch_bounds__(256) k_fold_coeffs(const double *__restrict__ 
 // contributor's four coefficients are formed on the way, in the operations of the
 // spline build, so W has the same bits while a quarter of the bytes is read (the
 // coefficients are neither written nor read).  A thread takes one key through kFoldRun
-// segments, whose inner knots it reads once.  Bound by the latency of the rows' loads:
+// segments, whose inner knots it reads once.  A one-dimensional grid, the key tiles of
+// a run of segments together: any number of segments, and rows that two tiles read are
+// in L2 for the second.  Bound by the latency of the rows' loads:
 // one year, 3843 modes: 61 us (112 us from the coefficients; 65 us a segment at a
 // time, 63 us by four).
 constexpr int kFoldRun = 2;
@@ -94,11 +96,11 @@ __global__ void __launch_bounds__(128, 5) k_fold_slopes(const double2 *__restric
                                                         const double2 *__restrict__ ylms,
                                                         const int *__restrict__ key_ptr,
                                                         const int *__restrict__ key_list, int K, int nseg, int nkeys,
-                                                        double2 *__restrict__ W)
+                                                        int tiles, double2 *__restrict__ W)
 {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    const int run = blockIdx.x / tiles, q = (blockIdx.x - run * tiles) * blockDim.x + threadIdx.x;
     if (q >= nkeys) return;
-    const int s0 = blockIdx.y * kFoldRun, n = min(kFoldRun, nseg - s0);
+    const int s0 = run * kFoldRun, n = min(kFoldRun, nseg - s0);
     double2 acc[kFoldRun][4];
     double ih[kFoldRun];
 #pragma unroll
@@ -625,10 +627,11 @@ extern "C" int few_fold_slopes(const void *y, const void *slopes, const double *
         return few::fail(FEW_ERR_SIZE, "few_fold_slopes: bad sizes");
     if (nseg == 0) return FEW_OK;
     const int nkeys = R * NN;
-    dim3 grid((nkeys + 127) / 128, (nseg + few::kFoldRun - 1) / few::kFoldRun);
-    if (grid.y > 65535) return few::fail(FEW_ERR_SIZE, "few_fold_slopes: %d segments are too many", nseg);
-    few::k_fold_slopes<<<grid, 128, 0, (cudaStream_t)stream>>>(
-        (const double2 *)y, (const double2 *)slopes, fac, (const double2 *)ylms, key_ptr, key_list, K, nseg, nkeys,
+    const int tiles = (nkeys + 127) / 128;
+    const long long blocks = (long long)((nseg + few::kFoldRun - 1) / few::kFoldRun) * tiles;
+    if (blocks > 0x7fffffffLL) return few::fail(FEW_ERR_SIZE, "few_fold_slopes: %d segments of %d keys are too many", nseg, nkeys);
+    few::k_fold_slopes<<<(unsigned)blocks, 128, 0, (cudaStream_t)stream>>>(
+        (const double2 *)y, (const double2 *)slopes, fac, (const double2 *)ylms, key_ptr, key_list, K, nseg, nkeys, tiles,
         (double2 *)W);
     FEW_LAUNCH_CHECK("k_fold_slopes");
     return FEW_OK;
