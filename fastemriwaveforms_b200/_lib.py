@@ -40,6 +40,8 @@ SIGNATURES = {
     "few_spline_build_factored": [_vp, _vp, _c_ll, _c_ll, _c_int, _c_ll, _c_int, _c_int, _vp, _c_int, _vp],
     "few_spline_overlap": [_vp, _c_int],
     "few_spline_max_overlap": [],
+    "few_spline_joined_scratch": [_c_int, _c_int],
+    "few_spline_build_joined": [_vp, _c_int, _vp, _c_ll, _c_ll, _c_int, _c_ll, _c_int, _c_int, _vp, _c_int, _vp, _vp],
     "few_spline_build_chunked": [_vp, _c_int, _vp, _c_ll, _c_ll, _c_int, _c_ll, _c_int, _c_int, _vp, _c_int, _vp],
     "few_spline_slopes": [_vp, _vp, _c_int, _c_int, _vp, _vp],
     "few_fold_slopes": [_vp, _vp, _vp, _vp, _vp, _vp, _c_int, _c_int, _c_int, _c_int, _c_int, _vp, _vp],
@@ -107,7 +109,8 @@ SIGNATURES = {
                             _c_int, _vp, _c_int, _c_int, _c_int, _vp],
 }
 _RESTYPE = {"few_last_error": ctypes.c_char_p, "few_mixed_operand_bytes": ctypes.c_longlong,
-            "few_mixed_adjoint_operand_bytes": ctypes.c_longlong, "few_adjoint_joint_scratch": ctypes.c_longlong}
+            "few_mixed_adjoint_operand_bytes": ctypes.c_longlong, "few_adjoint_joint_scratch": ctypes.c_longlong,
+            "few_spline_joined_scratch": ctypes.c_longlong}
 
 _lock = threading.Lock()
 _lib = None

@@ -222,17 +222,19 @@ int spline_factor(const double *x, int N, double *fac)
 
 // Rows after which the sweeps of the factorization have forgotten their start: the
 // smallest w such that every product of w successive factors, forward (-lo_i/den_i)
-// and backward (-c'_i), is below 2^-60.  Large when some knots are very uneven.
+// and backward (-c'_i), is below 2^-70.  37 on even knots, whose factors are 2 - sqrt(3);
+// over thousands of random, geometric, alternating and wandering knots 55 at most.
 int spline_overlap(const double *fac, int N)
 {
     if (!fac) return fail(FEW_ERR_ARG, "few_spline_overlap: null pointer");
     if (N < 4) return fail(FEW_ERR_SIZE, "few_spline_overlap: length=%d < 4", N);
     const int W = kFacWidth;
-    const double tol = 0x1p-60;
+    const double tol = 0x1p-70;
     int w = 1;
     for (int way = 0; way < 2; ++way) {
-        // runs [a, i) of factors whose product is just below tol, by two ends; a zero
-        // factor (the first row, or the last) ends every run across it
+        // runs [a, i] of factors whose product is just below tol, or not yet (one more is
+        // needed then), by two ends; a zero factor (the first row, or the last) ends every
+        // run across it
         int a = 1;
         double p = 1.0;
         for (int i = 1; i <= N - 2; ++i) {
@@ -250,7 +252,7 @@ int spline_overlap(const double *fac, int N)
                 p /= g;
                 ++a;
             }
-            w = std::max(w, i - a + 1);
+            w = std::max(w, i - a + (p < tol ? 1 : 2));
         }
     }
     return w;

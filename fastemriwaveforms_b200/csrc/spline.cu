@@ -345,17 +345,23 @@ __global__ void __launch_bounds__(kRowThreads) k_spline_build_rows(SplineArgs a)
 // from the factor table; the sweep temporaries are parked in the c3 output
 // row, which the last pass overwrites.  Loads are issued kSweepBatch steps
 // ahead of the arithmetic that uses them.
-constexpr int kSweepBatch = 8;
-
 //
 // COEF = false stores the slopes alone, s[i * ni + series] (the same bits as the c1
 // plane): a consumer that forms the coefficients from (y, s) spares three of the four
 // planes' writes and reads, and the sweep temporaries then stay in L2.  7686 series of
 // 1000 knots: 66 us, 122 us with the coefficients.
-template <bool COEF>
+//
+// CHECK: `out` holds what k_spline_chunks built with `overlap`; a CTA whose 32 series'
+// records chk say that nothing was left out that shows returns at once (3 us for 256
+// series of 1000 knots).
+constexpr int kSweepBatch = 8;
+constexpr int kChunkRows = 32;
+
+template <bool COEF, bool CHECK>
 __global__ void __launch_bounds__(32 * kScanChunks) k_spline_build_factored(
     const double *__restrict__ fac, const double *__restrict__ y, long long sk, long long sp, int split,
-    long long off2, int ni, int N, double *__restrict__ out, long long os_i, long long os_p)
+    long long off2, int ni, int N, double *__restrict__ out, long long os_i, long long os_p,
+    const double *__restrict__ chk, int overlap)
 {
     constexpr int W = kFacWidth;
     constexpr int P = kScanChunks;
@@ -371,6 +377,20 @@ __global__ void __launch_bounds__(32 * kScanChunks) k_spline_build_factored(
     double *o1 = o0 + plane;
     double *o2 = o1 + plane;
     double *o3 = COEF ? o2 + plane : o0;  // the sweep temporaries, then c3 (or the slopes)
+    if (CHECK) {
+        const int chunks = (N - 2 + kChunkRows - 1) / kChunkRows;
+        bool anew = false;
+        for (int c = w; c < chunks; c += P) {
+            const int ca = 1 + c * kChunkRows, ce = min(ca + kChunkRows, N - 1);
+            const int before = ca - overlap - 1;    // the row whose state the forward sweep left out; none below 1
+            const long long after = ce + overlap;   // and the backward one; none from N - 1 on
+            const double *lim = chk + (long long)c * 3 * ni + p;
+            if (before >= 1)
+                anew |= !(fabs(chk[(long long)((before - 1) / kChunkRows) * 3 * ni + p]) <= lim[ni]);
+            if (after < N - 1) anew |= !(fabs(o1[after * os_i]) <= lim[2LL * ni]);
+        }
+        if (!__syncthreads_or(anew)) return;
+    }
     const int L = (N - 2 + P - 1) / P;
     const int a = 1 + w * L, e = min(a + L, N - 1);  // this warp's rows [a, e); empty if a >= e
 
@@ -555,14 +575,23 @@ __global__ void __launch_bounds__(32 * kScanChunks) k_spline_build_factored(
 
 // Shared-knot build in one pass, for knots whose sweeps forget their start within
 // `overlap` rows (few_spline_overlap: every product of that many factors is below
-// 2^-60).  A warp takes 32 series (lane = series) and a chunk of kChunkRows rows: it
+// 2^-70).  A warp takes 32 series (lane = series) and a chunk of kChunkRows rows: it
 // sweeps forward from `overlap` rows before the chunk to `overlap` rows past it and
 // backward over the chunk, so no carries are exchanged and nothing but y is read from
 // memory; the forward values of the chunk stay in shared memory, a column per
-// thread.  The neighbouring chunks' rows read again are in L2.  Bound by the writes
-// (2048 series of 2000 knots: 102 us, 148 us in scan form) or, for few series, by the
-// chain of a chunk and its overlaps (256 series of 1000 knots: 16 us, 67 us).
-constexpr int kChunkRows = 32;
+// thread.  The neighbouring chunks' rows read again are in L2.
+//
+// What a chunk leaves out is the share of the sweeps' states at its far ends, a product
+// of `overlap` factors times the state.  For most data that is below any rounding here,
+// but not for every value: a NaN or an infinity reaches every knot of its series, and
+// beside values 2^17 times smaller the share of a large one shows.  So each chunk
+// records how large these states may be for their shares to stay within a rounding of
+// what is added up here (chk: the state that another chunk left out, and the limits for
+// its own two), and k_spline_build_factored<true, true> then compares them with the
+// states that the other chunks came to, and builds the 32 series anew in scan form where
+// one is larger or not a number.  Bound by the writes (2048 series of 2000 knots: 116 us
+// with the comparison, 148 us in scan form) or, for few series, by the chain of a chunk
+// and its overlaps (256 series of 1000 knots: 23 us, 67 us).
 constexpr int kChunkWarps = 4;
 constexpr int kMaxOverlap = 96;
 constexpr int kAhead = 8;  // rows whose loads are in flight ahead of the sweep
@@ -574,7 +603,18 @@ struct ChunkArgs {
     int split, ni, N, overlap;
     double *out;
     long long os_i, os_p;
+    double *chk;  // (chunks, 3, ni)
+    int groups;   // of 32 series
 };
+
+__host__ __device__ inline int spline_chunks(int N) { return (N - 2 + kChunkRows - 1) / kChunkRows; }
+
+// Limit of a left-out state whose share is `share` of it, beside a sum of size `sum`.
+__device__ __forceinline__ double state_limit(double sum, double share)
+{
+    const double v = 0x1p-53 * sum / share;
+    return v > 1.7976931348623157e308 ? 1.7976931348623157e308 : v;  // NaN stays; an infinite state is over any limit
+}
 
 // Row i of the factorization as the sweeps use it:
 // r'_i = A r'_{i-1} + alpha delta_{i-1} + beta delta_i, s_i = r'_i + C s_{i+1}.
@@ -590,7 +630,8 @@ __global__ void __launch_bounds__(32 * kChunkWarps) k_spline_chunks(ChunkArgs A)
     const int tid = threadIdx.x, lane = tid & 31;
     const int N = A.N, ni = A.ni, ov = A.overlap;
     const double *__restrict__ fac = A.fac;
-    const int a0 = 1 + blockIdx.y * kChunkWarps * kChunkRows;
+    const int tile = blockIdx.x / A.groups, group = blockIdx.x - tile * A.groups;
+    const int a0 = 1 + tile * kChunkWarps * kChunkRows;
     const int t0 = max(0, a0 - ov - 1), t1 = min(a0 + kChunkWarps * kChunkRows + ov, N - 1);  // rows [t0, t1) of the table
     for (int i = t0 + tid; i < t1; i += T) {
         const double *g = fac + (long long)W * i;
@@ -601,9 +642,10 @@ __global__ void __launch_bounds__(32 * kChunkWarps) k_spline_chunks(ChunkArgs A)
     const ChunkRow *row = tab - t0;
     const int a = a0 + (tid >> 5) * kChunkRows, e = min(a + kChunkRows, N - 1);
     if (a >= e) return;
-    const int p0 = blockIdx.x * 32 + lane;
+    const int p0 = group * 32 + lane;
     const bool live = p0 < ni;
     const int p = live ? p0 : ni - 1;  // idle lanes compute on a valid series and store nothing
+    double *chk = A.chk + (long long)(a - 1) / kChunkRows * 3 * ni + p;
     const double *__restrict__ yb =
         (p < A.split) ? A.y + (long long)p * A.sp : A.y + A.off2 + (long long)(p - A.split) * A.sp;
     const long long sk = A.sk;
@@ -614,7 +656,8 @@ __global__ void __launch_bounds__(32 * kChunkWarps) k_spline_chunks(ChunkArgs A)
     const int b = max(1, a - ov), f = min(e + ov, N - 1);
     double s_next = 0.0;  // s_e, then s_{i+1} of the backward sweep
     {
-        double prod = 1.0;
+        double prod = 1.0, before = 1.0;         // shares of s_f and r'_{b-1}
+        double sum_s = 0.0, sum_r = 0.0;         // what s_e and r'_{a-1} are added up from, by size
         double r = 0.0, ym = yb[(long long)b * sk];
         double dprev = (ym - yb[(long long)(b - 1) * sk]) * row[b - 1].ih;
         double ahead[kAhead];
@@ -640,12 +683,22 @@ __global__ void __launch_bounds__(32 * kChunkWarps) k_spline_chunks(ChunkArgs A)
                     r = fma(row[i].A, r, u[q]);
                     if (i >= e) {
                         s_next = fma(prod, r, s_next);
+                        sum_s = fma(fabs(prod), fabs(r), sum_s);
                         prod *= row[i].C;
                     } else if (i >= a) {
                         col[(i - a) * T] = r;
+                        // the state before the first row of a later chunk's forward sweep
+                        if ((i + ov) % kChunkRows == 0 && live) chk[0] = r;
+                    } else {
+                        sum_r = fma(fabs(row[i].A), sum_r, fabs(u[q]));
+                        before *= row[i].A;
                     }
                 }
             }
+        }
+        if (live) {
+            chk[ni] = state_limit(sum_r, fabs(before));
+            chk[2LL * ni] = state_limit(sum_s, fabs(prod));
         }
     }
     // backward sweep over rows [a, e): the slopes
@@ -721,15 +774,18 @@ __global__ void __launch_bounds__(32 * kChunkWarps) k_spline_chunks(ChunkArgs A)
     }
 }
 
-int launch_spline_chunks(const ChunkArgs &a, cudaStream_t st)
+int launch_spline_chunks(ChunkArgs a, cudaStream_t st)
 {
     constexpr int T = 32 * kChunkWarps;
-    const int rows = a.N - 2, chunks = (rows + kChunkRows - 1) / kChunkRows;
-    const int smem = std::min(rows, kChunkRows) * T * 8;
-    dim3 grid((a.ni + 31) / 32, (chunks + kChunkWarps - 1) / kChunkWarps);
-    if (grid.y > 65535) return fail(FEW_ERR_SIZE, "spline build: %d knots are too many", a.N);
-    k_spline_chunks<<<grid, T, smem, st>>>(a);
+    const int smem = std::min(a.N - 2, kChunkRows) * T * 8;
+    a.groups = (a.ni + 31) / 32;
+    const long long blocks = (long long)((spline_chunks(a.N) + kChunkWarps - 1) / kChunkWarps) * a.groups;
+    if (blocks > 0x7fffffffLL) return fail(FEW_ERR_SIZE, "spline build: %d series of %d knots are too many", a.ni, a.N);
+    k_spline_chunks<<<(unsigned)blocks, T, smem, st>>>(a);
     FEW_LAUNCH_CHECK("k_spline_chunks");
+    k_spline_build_factored<true, true><<<a.groups, 32 * kScanChunks, 0, st>>>(
+        a.fac, a.y, a.sk, a.sp, a.split, a.off2, a.ni, a.N, a.out, a.os_i, a.os_p, a.chk, a.overlap);
+    FEW_LAUNCH_CHECK("k_spline_build_factored");
     return FEW_OK;
 }
 
@@ -905,30 +961,52 @@ extern "C" int few_spline_build_factored(const double *fac, const double *y, lon
     if (y_split < 0 || y_split > ninterps) return few::fail(FEW_ERR_ARG, "few_spline_build_factored: bad y_split");
     const long long os_i = layout == FEW_LAYOUT_KNOT_MAJOR ? ninterps : 1;
     const long long os_p = layout == FEW_LAYOUT_KNOT_MAJOR ? 1 : length;
-    few::k_spline_build_factored<true><<<(ninterps + 31) / 32, 32 * few::kScanChunks, 0, (cudaStream_t)stream>>>(
-        fac, y, y_knot_stride, y_interp_stride, y_split, y_split_offset, ninterps, length, coeffs, os_i, os_p);
+    few::k_spline_build_factored<true, false><<<(ninterps + 31) / 32, 32 * few::kScanChunks, 0, (cudaStream_t)stream>>>(
+        fac, y, y_knot_stride, y_interp_stride, y_split, y_split_offset, ninterps, length, coeffs, os_i, os_p, nullptr, 0);
     FEW_LAUNCH_CHECK("k_spline_build_factored");
     return FEW_OK;
 }
 
 extern "C" int few_spline_max_overlap(void) { return few::kMaxOverlap; }
 
+extern "C" long long few_spline_joined_scratch(int ninterps, int length)
+{
+    return ninterps < 1 || length < 4 ? 0 : 3LL * few::spline_chunks(length) * ninterps;
+}
+
+extern "C" int few_spline_build_joined(const double *fac, int overlap, const double *y, long long y_knot_stride,
+                                       long long y_interp_stride, int y_split, long long y_split_offset, int ninterps,
+                                       int length, double *coeffs, int layout, double *scratch, void *stream)
+{
+    few::clear_error();
+    if (!fac || !y || !coeffs || !scratch) return few::fail(FEW_ERR_ARG, "few_spline_build_joined: null pointer");
+    if (ninterps < 1) return few::fail(FEW_ERR_SIZE, "few_spline_build_joined: ninterps=%d < 1", ninterps);
+    if (length < 4) return few::fail(FEW_ERR_SIZE, "few_spline_build_joined: length=%d < 4", length);
+    if (overlap < 1 || overlap > few::kMaxOverlap)
+        return few::fail(FEW_ERR_SIZE, "few_spline_build_joined: overlap=%d out of 1..%d", overlap, few::kMaxOverlap);
+    if (layout != FEW_LAYOUT_KNOT_MAJOR && layout != FEW_LAYOUT_INTERP_MAJOR)
+        return few::fail(FEW_ERR_ARG, "few_spline_build_joined: unknown layout %d", layout);
+    if (y_split < 0 || y_split > ninterps) return few::fail(FEW_ERR_ARG, "few_spline_build_joined: bad y_split");
+    few::ChunkArgs a{fac, y, y_knot_stride, y_interp_stride, y_split_offset, y_split, ninterps, length, overlap, coeffs,
+                     layout == FEW_LAYOUT_KNOT_MAJOR ? ninterps : 1, layout == FEW_LAYOUT_KNOT_MAJOR ? 1 : length,
+                     scratch, 0};
+    return few::launch_spline_chunks(a, (cudaStream_t)stream);
+}
+
 extern "C" int few_spline_build_chunked(const double *fac, int overlap, const double *y, long long y_knot_stride,
                                         long long y_interp_stride, int y_split, long long y_split_offset, int ninterps,
                                         int length, double *coeffs, int layout, void *stream)
 {
     few::clear_error();
-    if (!fac || !y || !coeffs) return few::fail(FEW_ERR_ARG, "few_spline_build_chunked: null pointer");
     if (ninterps < 1) return few::fail(FEW_ERR_SIZE, "few_spline_build_chunked: ninterps=%d < 1", ninterps);
     if (length < 4) return few::fail(FEW_ERR_SIZE, "few_spline_build_chunked: length=%d < 4", length);
-    if (overlap < 1 || overlap > few::kMaxOverlap)
-        return few::fail(FEW_ERR_SIZE, "few_spline_build_chunked: overlap=%d out of 1..%d", overlap, few::kMaxOverlap);
-    if (layout != FEW_LAYOUT_KNOT_MAJOR && layout != FEW_LAYOUT_INTERP_MAJOR)
-        return few::fail(FEW_ERR_ARG, "few_spline_build_chunked: unknown layout %d", layout);
-    if (y_split < 0 || y_split > ninterps) return few::fail(FEW_ERR_ARG, "few_spline_build_chunked: bad y_split");
-    few::ChunkArgs a{fac, y, y_knot_stride, y_interp_stride, y_split_offset, y_split, ninterps, length, overlap, coeffs,
-                     layout == FEW_LAYOUT_KNOT_MAJOR ? ninterps : 1, layout == FEW_LAYOUT_KNOT_MAJOR ? 1 : length};
-    return few::launch_spline_chunks(a, (cudaStream_t)stream);
+    cudaStream_t st = (cudaStream_t)stream;
+    void *scratch = nullptr;
+    FEW_CUDA_TRY(cudaMallocAsync(&scratch, (size_t)few_spline_joined_scratch(ninterps, length) * 8, st));
+    const int rc = few_spline_build_joined(fac, overlap, y, y_knot_stride, y_interp_stride, y_split, y_split_offset,
+                                           ninterps, length, coeffs, layout, static_cast<double *>(scratch), stream);
+    FEW_CUDA_TRY(cudaFreeAsync(scratch, st));
+    return rc;
 }
 
 extern "C" int few_spline_slopes(const double *fac, const double *y, int ninterps, int length, double *slopes,
@@ -938,8 +1016,8 @@ extern "C" int few_spline_slopes(const double *fac, const double *y, int ninterp
     if (!fac || !y || !slopes) return few::fail(FEW_ERR_ARG, "few_spline_slopes: null pointer");
     if (ninterps < 1) return few::fail(FEW_ERR_SIZE, "few_spline_slopes: ninterps=%d < 1", ninterps);
     if (length < 4) return few::fail(FEW_ERR_SIZE, "few_spline_slopes: length=%d < 4", length);
-    few::k_spline_build_factored<false><<<(ninterps + 31) / 32, 32 * few::kScanChunks, 0, (cudaStream_t)stream>>>(
-        fac, y, ninterps, 1, ninterps, 0, ninterps, length, slopes, ninterps, 1);
+    few::k_spline_build_factored<false, false><<<(ninterps + 31) / 32, 32 * few::kScanChunks, 0, (cudaStream_t)stream>>>(
+        fac, y, ninterps, 1, ninterps, 0, ninterps, length, slopes, ninterps, 1, nullptr, 0);
     FEW_LAUNCH_CHECK("k_spline_build_factored");
     return FEW_OK;
 }

@@ -171,10 +171,15 @@ def _ptr(t: torch.Tensor) -> int:
     return t.data_ptr()
 
 
-# From this many knots on, the one-pass spline builds are the faster ones (below, the
-# chunks of k_spline_build_factored are shorter than a run and its overlaps: 8.1
-# against 10.8 us at 100 knots of 400 series, 13.4 against 11.4 us at 200).
-ONE_PASS_KNOTS = 150
+# The spline build over independent runs of knots (few_spline_build_joined) is taken from
+# ONE_PASS_KNOTS on, and for more series than MANY_SERIES, which fill the chip in scan
+# form (few_spline_build_factored) as well, from MANY_KNOTS on.  us on B200 in scan form
+# and over runs: 64 series of 300 knots 16.8 and 18.3, of 350 19.3 and 18.7, of 700 35 and
+# 20; 3000 of 350 20 and 22, of 700 37 and 32; 4096 of 700 37 and 49; 7686 of 700 68 and
+# 82, of 1000 115 and 108, of 2000 275 and 197.
+ONE_PASS_KNOTS = 350
+MANY_SERIES = 3000
+MANY_KNOTS = 1000
 
 
 def spline_factor_host(h_t: np.ndarray) -> np.ndarray:
@@ -187,7 +192,7 @@ def spline_factor_host(h_t: np.ndarray) -> np.ndarray:
 
 def spline_factor(h_t: np.ndarray, device):
     """Device copy of the factorization for knots h_t, and its overlap
-    (few_spline_overlap; 0 where the one-pass builds are not used)."""
+    (few_spline_overlap; 0 where the build over runs is not used)."""
     fac, N = spline_factor_host(h_t), len(h_t)
     overlap = 0
     if N >= ONE_PASS_KNOTS:
@@ -206,9 +211,11 @@ def spline_factor_table(h_t: np.ndarray, device) -> torch.Tensor:
 def build_splines(fac, overlap, y_ptr, y_strides, ninterps, length, coeffs, st):
     """Spline coefficients (4, length, ninterps) on shared knots; y_strides =
     (knot stride, series stride, split, split offset) of few_spline_build."""
-    if overlap:
-        _lib.call("few_spline_build_chunked", _ptr(fac), overlap, y_ptr, *y_strides, ninterps, length, _ptr(coeffs),
-                  _lib.FEW_LAYOUT_KNOT_MAJOR, st)
+    if overlap and (ninterps <= MANY_SERIES or length >= MANY_KNOTS):
+        scratch = torch.empty(int(_lib.load().few_spline_joined_scratch(ninterps, length)), dtype=torch.float64,
+                              device=coeffs.device)
+        _lib.call("few_spline_build_joined", _ptr(fac), overlap, y_ptr, *y_strides, ninterps, length, _ptr(coeffs),
+                  _lib.FEW_LAYOUT_KNOT_MAJOR, _ptr(scratch), st)
     else:
         _lib.call("few_spline_build_factored", _ptr(fac), y_ptr, *y_strides, ninterps, length, _ptr(coeffs),
                   _lib.FEW_LAYOUT_KNOT_MAJOR, st)

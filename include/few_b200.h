@@ -168,14 +168,24 @@ FEW_API int few_spline_build_factored(const double *fac, const double *y, long l
 
 /* Rows after which the sweeps of a factorization fac [host] (few_spline_factor, N
  * knots) have forgotten their start: every product of that many of their factors is
- * below 2^-60 (30 to 40 on ordinary knots).  Negative: an error status. */
+ * below 2^-70 (35 to 55 on ordinary knots).  Negative: an error status. */
 FEW_API int few_spline_overlap(const double *fac, int N);
 
-/* Largest overlap few_spline_build_chunked takes. */
+/* Largest overlap few_spline_build_joined takes. */
 FEW_API int few_spline_max_overlap(void);
 
-/* few_spline_build_factored in one pass over independent runs of knots, for
- * 1 <= overlap <= few_spline_max_overlap() (few_spline_overlap's, or more). */
+/* few_spline_build_factored over independent runs of knots, for
+ * 1 <= overlap <= few_spline_max_overlap() (few_spline_overlap's, or more).  What the
+ * runs' ends leave out is compared with what they add up; where it would show (values
+ * many orders of magnitude apart, or not finite) the series and those built with it get
+ * few_spline_build_factored's own bits.  scratch [device]:
+ * few_spline_joined_scratch(ninterps, length) doubles. */
+FEW_API int few_spline_build_joined(const double *fac, int overlap, const double *y, long long y_knot_stride,
+                                    long long y_interp_stride, int y_split, long long y_split_offset, int ninterps,
+                                    int length, double *coeffs, int layout, double *scratch, void *stream);
+FEW_API long long few_spline_joined_scratch(int ninterps, int length);
+
+/* The same with scratch from the device's stream-ordered pool. */
 FEW_API int few_spline_build_chunked(const double *fac, int overlap, const double *y, long long y_knot_stride,
                                      long long y_interp_stride, int y_split, long long y_split_offset, int ninterps,
                                      int length, double *coeffs, int layout, void *stream);
