@@ -61,11 +61,18 @@ __device__ __forceinline__ void write_segment(double *o1, double *o2, double *o3
     o3[off] = tt / dx;
 }
 
+// What k_spline_build_rows leaves in place of the first slope of a series that it gives up
+// (a NaN's bits: a series that happens to have them is built twice, alike).
+constexpr long long kGivenUp = 0x7ff8b2005eed0001LL;
+
+// MARKED: only the series that k_spline_build_rows has given up.
+template <bool MARKED>
 __global__ void __launch_bounds__(128) k_spline_build(SplineArgs a)
 {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= a.ni) return;
     const int N = a.N;
+    if (MARKED && __double_as_longlong(a.out[(long long)p * a.os_p + (long long)N * a.ni]) != kGivenUp) return;
     const double *x = a.t + (long long)p * a.t_rs;
     const double *yb = (p < a.split) ? a.y + (long long)p * a.sp : a.y + a.off2 + (long long)(p - a.split) * a.sp;
     const long long sk = a.sk;
@@ -160,9 +167,10 @@ __global__ void __launch_bounds__(128) k_spline_build(SplineArgs a)
 // So each thread takes one run of rows and starts kWarmup rows before it from an
 // arbitrary state; the threads then compare the state they came to at their first
 // row with the one the thread before ended with, and only if all agree to the
-// last bit is the result that of the serial sweep; otherwise one thread sweeps
-// the series (two sweeps that differ by 1e-25 agree in every bit, so this is not
-// seen in use).  Knots, right-hand sides and sweep values stay in shared memory;
+// last bit is the result that of the serial sweep.  Sweeps that differ by 1e-25 of
+// themselves agree in every bit, but the state behind a pulse, a step or a NaN does not:
+// then one thread sweeps the series, or (give_up: more series than a few at a time on an
+// SM, where that would take longer) it is left to the thread form.  Knots, right-hand sides and sweep values stay in shared memory;
 // everything else is formed with consecutive knots on consecutive threads.  Bound
 // by the chain of 64 + N/128 steps: 34 us for 3 series of 1000 knots and 46 us for
 // 256 (592 and 800 us with a thread per series); with a warp per series and the
@@ -215,7 +223,7 @@ __device__ __forceinline__ bool same_bits(double a, double b)
     return __double_as_longlong(a) == __double_as_longlong(b);
 }
 
-__global__ void __launch_bounds__(kRowThreads) k_spline_build_rows(SplineArgs a)
+__global__ void __launch_bounds__(kRowThreads) k_spline_build_rows(SplineArgs a, bool give_up)
 {
     extern __shared__ __align__(16) double row_smem[];
     __shared__ double s_c[kRowThreads + 1], s_r[kRowThreads + 1];
@@ -271,6 +279,10 @@ __global__ void __launch_bounds__(kRowThreads) k_spline_build_rows(SplineArgs a)
     s_r[tid + 1] = r;
     __syncthreads();
     if (__syncthreads_or(has && tid > 0 && !(same_bits(ck, s_c[tid]) && same_bits(rk, s_r[tid])))) {
+        if (give_up) {
+            if (tid == 0) o1[0] = __longlong_as_double(kGivenUp);
+            return;
+        }
         c = r = 0.0;
         if (tid == 0) forward_rows(w, 1, 1, N - 1, c, r, ck, rk);
         __syncthreads();
@@ -292,6 +304,10 @@ __global__ void __launch_bounds__(kRowThreads) k_spline_build_rows(SplineArgs a)
     s_c[tid] = s;
     __syncthreads();
     if (__syncthreads_or(has && last < N - 1 && !same_bits(s_in, s_c[tid + 1]))) {
+        if (give_up) {
+            if (tid == 0) o1[0] = __longlong_as_double(kGivenUp);
+            return;
+        }
         if (tid == 0) {
             s = w.rp[N - 2];
             slope[N - 2] = s;
@@ -931,17 +947,26 @@ int launch_spline_build(const double *t, long long t_rs, const double *y, long l
     }
     const int threads = 128;
     const size_t smem = (size_t)4 * N * sizeof(double);
-    // A CTA per series until the thread form has enough series to fill the chip:
-    // it takes 0.6-0.8 us a knot whatever their number, the CTAs 8, 22, 36 and 300
-    // ns a series at 12, 50, 200 and 2000 knots.
-    if (ni <= 1024 + 3LL * N && smem <= kRowSmem) {
+    // A CTA per series until the thread form has enough series to fill the chip: it takes
+    // 0.8-1.3 us a knot whatever their number, the CTAs 8, 22, 36, 130, 280, 610 and 600 ns
+    // a series at 12, 50, 200, 1000, 2000, 4000 and 6000 knots.  Series that the CTAs give
+    // up are better swept there, one thread each, while few go to an SM: 256 pulses of
+    // 1000 knots 422 us (thread form 2060), 400 of 6000 6.9 ms (12.5); 5000 of 4000 knots
+    // 12.5 ms given up and 52 ms swept there (9.8).
+    if (ni <= std::min(1024 + 3LL * N, 8000LL) && smem <= kRowSmem) {
+        const int per_sm = std::min(16, 228 * 1024 / ((int)smem + 3328));
+        const bool give_up = ni > 3 * 148 * per_sm;
         FEW_CUDA_TRY(ensure_smem_attr((const void *)k_spline_build_rows, kRowSmem));
-        k_spline_build_rows<<<ni, kRowThreads, smem, st>>>(a);
+        k_spline_build_rows<<<ni, kRowThreads, smem, st>>>(a, give_up);
         FEW_LAUNCH_CHECK("k_spline_build_rows");
+        if (give_up) {
+            k_spline_build<true><<<(ni + threads - 1) / threads, threads, 0, st>>>(a);
+            FEW_LAUNCH_CHECK("k_spline_build");
+        }
         return FEW_OK;
     }
     const int blocks = (ni + threads - 1) / threads;
-    k_spline_build<<<blocks, threads, 0, st>>>(a);
+    k_spline_build<false><<<blocks, threads, 0, st>>>(a);
     FEW_LAUNCH_CHECK("k_spline_build");
     return FEW_OK;
 }
