@@ -170,8 +170,9 @@ struct SumArgs {
     const int *row_m;
     const int *row_k;
     int N, R, nlo, NN;
-    int nblk;             // row blocks
-    int blocks_per_pass;  // of them, those whose coefficients are in shared memory at once
+    int nblk;             // row blocks; 0: ceil(R / RB), the usual count (as a value the kernel
+                          // knows: 6.53 ms against 6.58 at one year, 3843 modes, faithful)
+    int blocks_per_pass;  // of them, those whose coefficients are in shared memory at once (>= 1)
     int use_theta;
     double dt;
 };
@@ -321,7 +322,7 @@ __device__ __forceinline__ void sum_unit(const SumArgs &a, int seg, int lo, int 
                                          double *s_pc)
 {
     const double t0 = a.seg_info[3 * seg], pt0 = a.seg_info[3 * seg + 1], pw = a.seg_info[3 * seg + 2];
-    const int R = a.R, NN = a.NN, nlo = a.nlo, nblk = a.nblk;
+    const int R = a.R, NN = a.NN, nlo = a.nlo, nblk = a.nblk ? a.nblk : (R + RB - 1) / RB;
     const long long nps = (long long)(a.N - 1) * 3;
     const bool theta = THETA && a.use_theta;
     // The faithful form parks Phi_phi and e^{-i Phi_phi}, needed only at each
@@ -454,7 +455,8 @@ __global__ void __launch_bounds__(kSumThreads, (SPT == 1 || RB <= 4) ? 2 : 1) k_
         a.use_theta = d.use_theta;
         a.dt = d.dt;
         const SumBlocks sb = sum_blocks(d.R, d.NN, RB, smem_bytes);
-        a.nblk = sb.nblk;
+        if (sb.per_pass < 1) continue;  // not one row fits
+        a.nblk = sb.nblk == (d.R + RB - 1) / RB ? 0 : sb.nblk;
         a.blocks_per_pass = sb.per_pass;
         sum_unit<RB, FAITHFUL, SPT, true>(a, units4[4 * u + 1], units4[4 * u + 2], units4[4 * u + 3],
                                     reinterpret_cast<double2 *>(smem_raw), s_rm, s_rk, s_pc);
@@ -491,8 +493,8 @@ struct SumShape {
 // with 5, 7.06 at 8 x 1 and 4 x 1, 7.09 at 4 x 2); exact 6 x 1 4.20 ms (4.18 with 7,
 // 4.33 with 4, 4.33 at 8 x 2, 4.31 at 4 x 1 and 4.54 at 3 x 2 with neighbours), and
 // 0.88 ms on 363 modes with k' != 0 (R = 63, NN = 11; 0.89 with 7).  FP64 pipe 70 %
-// busy in the faithful form.  FEW_B200_SUM_SHAPE="RBxSPT" overrides both: 4 rows, or 8
-// for the most that there is.
+// busy in the faithful form.  FEW_B200_SUM_SHAPE overrides both with one of the shapes
+// that exist: "4x1", "4x2", or "8x1" and "8x2" for the most rows, 6 x 1 and 7 x 2.
 SumShape sum_shape(int mode)
 {
     static const SumShape forced = [] {
@@ -587,7 +589,7 @@ int launch_sum_folded(double2 *wf, const double2 *W, const double *pc, int N, co
     const SumShape sh = sum_shape(mode);
     const SumBlocks sb = sum_blocks(R, NN, sh.rb, kSmemBudget);
     if (sb.nblk < 1) return fail(FEW_ERR_SIZE, "few_sum_folded: NN=%d too large for one row in shared memory", NN);
-    a.nblk = sb.nblk;
+    a.nblk = sb.nblk == (R + sh.rb - 1) / sh.rb ? 0 : sb.nblk;
     a.blocks_per_pass = sb.per_pass;
     const size_t smem = (size_t)std::min(R, sb.per_pass * ((R + sb.nblk - 1) / sb.nblk)) * row_bytes;
     if (sh.rb == 4 && sh.spt == 2)
