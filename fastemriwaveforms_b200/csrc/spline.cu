@@ -999,19 +999,32 @@ extern "C" long long few_spline_joined_scratch(int ninterps, int length)
     return ninterps < 1 || length < 4 ? 0 : 3LL * few::spline_chunks(length) * ninterps;
 }
 
+namespace few {
+namespace {
+int check_joined(const char *who, const double *fac, int overlap, const double *y, int y_split, int ninterps, int length,
+                 const double *coeffs, int layout)
+{
+    clear_error();
+    if (!fac || !y || !coeffs) return fail(FEW_ERR_ARG, "%s: null pointer", who);
+    if (ninterps < 1) return fail(FEW_ERR_SIZE, "%s: ninterps=%d < 1", who, ninterps);
+    if (length < 4) return fail(FEW_ERR_SIZE, "%s: length=%d < 4", who, length);
+    if (overlap < 1 || overlap > kMaxOverlap)
+        return fail(FEW_ERR_SIZE, "%s: overlap=%d out of 1..%d", who, overlap, kMaxOverlap);
+    if (layout != FEW_LAYOUT_KNOT_MAJOR && layout != FEW_LAYOUT_INTERP_MAJOR)
+        return fail(FEW_ERR_ARG, "%s: unknown layout %d", who, layout);
+    if (y_split < 0 || y_split > ninterps) return fail(FEW_ERR_ARG, "%s: bad y_split", who);
+    return FEW_OK;
+}
+}  // namespace
+}  // namespace few
+
 extern "C" int few_spline_build_joined(const double *fac, int overlap, const double *y, long long y_knot_stride,
                                        long long y_interp_stride, int y_split, long long y_split_offset, int ninterps,
                                        int length, double *coeffs, int layout, double *scratch, void *stream)
 {
-    few::clear_error();
-    if (!fac || !y || !coeffs || !scratch) return few::fail(FEW_ERR_ARG, "few_spline_build_joined: null pointer");
-    if (ninterps < 1) return few::fail(FEW_ERR_SIZE, "few_spline_build_joined: ninterps=%d < 1", ninterps);
-    if (length < 4) return few::fail(FEW_ERR_SIZE, "few_spline_build_joined: length=%d < 4", length);
-    if (overlap < 1 || overlap > few::kMaxOverlap)
-        return few::fail(FEW_ERR_SIZE, "few_spline_build_joined: overlap=%d out of 1..%d", overlap, few::kMaxOverlap);
-    if (layout != FEW_LAYOUT_KNOT_MAJOR && layout != FEW_LAYOUT_INTERP_MAJOR)
-        return few::fail(FEW_ERR_ARG, "few_spline_build_joined: unknown layout %d", layout);
-    if (y_split < 0 || y_split > ninterps) return few::fail(FEW_ERR_ARG, "few_spline_build_joined: bad y_split");
+    const int rc = few::check_joined("few_spline_build_joined", fac, overlap, y, y_split, ninterps, length, coeffs, layout);
+    if (rc) return rc;
+    if (!scratch) return few::fail(FEW_ERR_ARG, "few_spline_build_joined: null pointer");
     few::ChunkArgs a{fac, y, y_knot_stride, y_interp_stride, y_split_offset, y_split, ninterps, length, overlap, coeffs,
                      layout == FEW_LAYOUT_KNOT_MAJOR ? ninterps : 1, layout == FEW_LAYOUT_KNOT_MAJOR ? 1 : length,
                      scratch, 0};
@@ -1022,14 +1035,13 @@ extern "C" int few_spline_build_chunked(const double *fac, int overlap, const do
                                         long long y_interp_stride, int y_split, long long y_split_offset, int ninterps,
                                         int length, double *coeffs, int layout, void *stream)
 {
-    few::clear_error();
-    if (ninterps < 1) return few::fail(FEW_ERR_SIZE, "few_spline_build_chunked: ninterps=%d < 1", ninterps);
-    if (length < 4) return few::fail(FEW_ERR_SIZE, "few_spline_build_chunked: length=%d < 4", length);
+    int rc = few::check_joined("few_spline_build_chunked", fac, overlap, y, y_split, ninterps, length, coeffs, layout);
+    if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
     void *scratch = nullptr;
     FEW_CUDA_TRY(cudaMallocAsync(&scratch, (size_t)few_spline_joined_scratch(ninterps, length) * 8, st));
-    const int rc = few_spline_build_joined(fac, overlap, y, y_knot_stride, y_interp_stride, y_split, y_split_offset,
-                                           ninterps, length, coeffs, layout, static_cast<double *>(scratch), stream);
+    rc = few_spline_build_joined(fac, overlap, y, y_knot_stride, y_interp_stride, y_split, y_split_offset, ninterps, length,
+                                 coeffs, layout, static_cast<double *>(scratch), stream);
     FEW_CUDA_TRY(cudaFreeAsync(scratch, st));
     return rc;
 }

@@ -43,3 +43,17 @@ def test_overlap(kind):
         products = [np.lib.stride_tricks.sliding_window_view(f, n).prod(axis=1).max() for n in (w, w - 2)
                     for f in factors]
         assert max(products[:2]) < 2.0**-70 <= max(products[2:]), (kind, N)
+
+
+def test_bad_arguments_are_refused_on_the_host():
+    import ctypes
+
+    lib = _lib.load()
+    d = ctypes.c_void_p(16)  # never read
+    for fn, tail in ((lib.few_spline_build_chunked, ()), (lib.few_spline_build_joined, (d,))):
+        call = lambda fac=d, ov=40, y=d, split=1, ni=1, n=400, out=d, layout=0: fn(  # noqa: E731
+            fac, ov, y, 1, 1, split, 0, ni, n, out, layout, *tail, None)
+        assert call(fac=None) == call(y=None) == call(out=None) == _lib.FEW_ERR_ARG
+        assert call(layout=2) == call(split=2) == _lib.FEW_ERR_ARG
+        assert call(ov=0) == call(ov=97) == call(ni=0) == call(n=3) == _lib.FEW_ERR_SIZE
+    assert lib.few_spline_build_joined(d, 40, d, 1, 1, 1, 0, 1, 400, d, 0, None, None) == _lib.FEW_ERR_ARG
