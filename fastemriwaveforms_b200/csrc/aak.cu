@@ -387,8 +387,9 @@ struct Harmonics {
 };
 
 // Bound by FP64 latency and issue at 16 warps per SM.  One year at dt = 10 s, 18
-// harmonics: 0.39 ms (2.02 ms with the nine recurrences, a sincos per harmonic and
-// the geometry's angles per sample), with the response 0.59 ms (2.17 ms).  A few
+// harmonics: 0.405 ms (2.02 ms with the nine recurrences, a sincos per harmonic and
+// the geometry's angles per sample), with the response 0.605 ms (2.17 ms); 0.39 and
+// 0.59 ms with plain sums on the way to powers of u, which lose digits.  A few
 // thousand samples of 24 harmonics: 16 us (41 us).
 template <int P, bool MICH>
 __global__ void __launch_bounds__(kThreads, 4) k_aak(AakArgs A) {
@@ -644,7 +645,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_aak(AakArgs A) {
 // Four samples a thread share each coefficient read, two with the response (whose
 // state for four spills: 0.60 against 0.59 ms at one year, 80 against 60 us at
 // 310,000 samples); one when more would leave SMs without a CTA.  Four CTAs per
-// SM: 0.39 ms plain at one year, 0.42 and 0.51 at three and two.
+// SM: with plain sums 0.39 ms at one year, 0.42 and 0.51 at three and two.
 int launch_aak(const AakArgs &A, int total, cudaStream_t st) {
     const int per = total < 148 * 2 * 4 * kThreads ? 1 : (A.mich ? 2 : 4);
     const int ctas = (total + per * kThreads - 1) / (per * kThreads);

@@ -744,8 +744,9 @@ __device__ __forceinline__ void fill_entry(const SumArgs &A, long long e, long l
     E.off = (int)(A.lo[e] + (base - A.prefix[e]));
 }
 
-// 1/sqrt(a) for a normal a: the hardware's approximation (20 bits) and one step
-// of the third-order iteration (error 2^-60 before rounding).
+// 1/sqrt(a) for a normal a: the hardware's approximation y (20 bits), then
+// a^(-1/2) = y (1 - e)^(-1/2) with e = 1 - a y^2 (|e| < 2^-19) by the binomial series to
+// e^2, whose next term, 5/16 e^3, is below 2^-58.
 __device__ __forceinline__ double rsqrt_pos(double a) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
@@ -893,10 +894,10 @@ __device__ __forceinline__ void fd_bins(const SumArgs &A, const Entry &E, const 
 // bin (the segment's ends, turnovers, small SPA arguments: 0.4 to 8 % of them)
 // takes the general path.
 // Bound by the FP64 pipe's latency and the shared-memory reads together (FP64
-// pipe 48 % busy, issue slots 59 % at 16 warps per SM).  One year, 3843 modes,
+// pipe 47 % busy, issue slots 58 % at 16 warps per SM).  One year, 3843 modes,
 // 889 million (mode, bin) evaluations: 14.75 ms (15.0 with the quadrant's signs by
 // negation and selection); 65.7 ms with every bin on the general path (1390
-// instructions a bin against about 320), 17.2 ms with one bin a lane, 26.1 ms at 8
+// instructions a bin against about 350), 17.2 ms with one bin a lane, 26.1 ms at 8
 // warps per SM.
 template <int MINB>
 __global__ void __launch_bounds__(kSumThreads, MINB) k_fd_sum(const __grid_constant__ SumArgs A) {

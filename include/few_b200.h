@@ -191,7 +191,8 @@ FEW_API int few_spline_build_chunked(const double *fac, int overlap, const doubl
                                      int length, double *coeffs, int layout, void *stream);
 
 /* The slopes at the knots of few_spline_build_factored's splines alone (the c1 plane,
- * same bits): y, slopes [device] (length, ninterps), not overlapping. */
+ * same bits, but for the last knot: here the system's own slope, there the last
+ * segment's derivative from its coefficients): y, slopes [device] (length, ninterps), not overlapping. */
 FEW_API int few_spline_slopes(const double *fac, const double *y, int ninterps, int length, double *slopes,
                               void *stream);
 
