@@ -114,11 +114,18 @@ def candidates_for(precision: str) -> list:
 
 
 def tune(key: str, make_runner, candidates) -> dict:
-    """Time make_runner(**shape)() for every candidate shape and cache the best."""
+    """Time make_runner(**shape)() for every candidate shape and cache the best.  Shapes
+    that the library refuses (an operand ring larger than shared memory: four B slots
+    beside two A stages from 40 rows on) are left out."""
     results = []
     for shape in candidates:
         run = make_runner(**shape)
-        results.append((time_ms(run), shape))
+        try:
+            results.append((time_ms(run), shape))
+        except ValueError as err:
+            refused = err
+    if not results:
+        raise refused
     results.sort(key=lambda r: r[0])
     best_ms, best = results[0]
     choice = dict(best, ms=best_ms, tried=[dict(sh, ms=t) for t, sh in results])
