@@ -493,8 +493,13 @@ struct SumShape {
 // with 5, 7.06 at 8 x 1 and 4 x 1, 7.09 at 4 x 2); exact 6 x 1 4.20 ms (4.18 with 7,
 // 4.33 with 4, 4.33 at 8 x 2, 4.31 at 4 x 1 and 4.54 at 3 x 2 with neighbours), and
 // 0.88 ms on 363 modes with k' != 0 (R = 63, NN = 11; 0.89 with 7).  FP64 pipe 70 %
-// busy in the faithful form.  FEW_B200_SUM_SHAPE overrides both with one of the shapes
-// that exist: "4x1", "4x2", or "8x1" and "8x2" for the most rows, 6 x 1 and 7 x 2.
+// busy in the faithful form.  Other row counts, a call of 500 knots and 1000000 samples
+// with blocks of up to 8 rows and a test per row, and now: faithful 5 rows 741 and 623 us,
+// 8 rows 1038 and 992, 9 rows 1266 and 1079, 15 rows 1851 and 1709, 16 rows 1959 and 1817,
+// 17 rows 2197 and 1921, 23 rows 2788 and 2569; exact (4 rows before) 5 rows 629 and 427, 8
+// rows 864 and 649, 15 rows 1539 and 1128, 23 rows 2303 and 1701.  FEW_B200_SUM_SHAPE
+// overrides both with one of the shapes that exist: "4x1", "4x2", or "8x1" and "8x2" for
+// the most rows, 6 x 1 and 7 x 2.
 SumShape sum_shape(int mode)
 {
     static const SumShape forced = [] {
